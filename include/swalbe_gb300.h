@@ -170,8 +170,10 @@ int swb_set_inclination(swb_state *s, double ax, double ay, int loop_time, int64
  * population loads and stores (the common steady τ = 1 step; other
  * iterations run as 64-thread strips of the same rows); or, with
  * nt = 32 (SWB_F32 / SWB_F16 only; h is ignored), CTAs of 256 threads own
- * 2D tiles of 32 x 16 cells whose loads are all issued at once.  By default
- * states autotune it on their first swb_step of >= 512 steps (timing a few
+ * 2D tiles of 32 x 16 cells whose loads are all issued at once.  SWB_F64
+ * states run one cell per thread whatever the geometry, which is only checked
+ * and kept.  By default
+ * the other states autotune it on their first swb_step of >= 512 steps (timing a few
  * geometries on those real steps; remembered per lattice size).  Setting it
  * (or (0, 0): a size rule) turns the autotuner off.  Results do not depend
  * on it: the per-cell arithmetic is the same in every form, and the mass that

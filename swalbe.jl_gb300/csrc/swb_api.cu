@@ -68,6 +68,22 @@ double incl_factor(long long t, long long tstart, long long tsmooth) {
     return 0.5 + 0.5 * std::tanh((double)(t - tstart) / (double)tsmooth);
 }
 
+// Buffers of the Float64 cell kernels: pressure, θ-wave columns, accumulators.
+size_t cell_bytes(const swb_params &p) {
+    return ((size_t)p.Lx * p.Ly + 2 * (size_t)p.Lx + 2 * swb::kAcc64) * 8;
+}
+
+// Key of the threshold t in the order the cell kernels compare heights in:
+// h > t iff h is no NaN and its key is larger (t + 0 makes -0 the zero that
+// no zero is above; nothing is above a NaN).
+unsigned long long threshold_key(double t) {
+    if (std::isnan(t)) return ~0ULL;
+    t += 0.0;
+    unsigned long long u;
+    memcpy(&u, &t, 8);
+    return (u >> 63) ? ~u : (u | 0x8000000000000000ULL);
+}
+
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 int real_bytes(int precision) { return precision == SWB_F64 || precision == SWB_PLAIN64 ? 8 : 4; }
@@ -185,8 +201,7 @@ bool launch_overlap() {
 
 cudaError_t launch_fused_step(int precision, const StepArgs &a, int k, bool steady, cudaStream_t st) {
     count_launches(1);
-    return precision == SWB_F64 ? launch_fused_step_f64(a, k, st)
-                                : launch_fused_step_f32(precision, a, k, steady, st);
+    return launch_fused_step_f32(precision, a, k, steady, st);
 }
 cudaError_t launch_moments(int precision, const StepArgs &a, cudaStream_t st) {
     count_launches(1);
@@ -289,6 +304,7 @@ struct swb_state {
     unsigned long long graph_launches = 0;  // kernels in the captured graph
     std::vector<void *> allocs;
     StepArgs a{};
+    swb::Cell64 x{};  // SWB_F64: the cell kernels' own buffers and constants
     PlainState ps{};
     double *plain_kapF = nullptr;
     double *plain_cosF = nullptr;  // cospi(θ) of a θ field (the plain path's measures)
@@ -433,11 +449,12 @@ __global__ void d2f_kernel(const double *src, float *dst, long long n) {
 }
 
 int set_fresh(swb_state *s) {
+    s->host_fresh = true;
+    s->fields_current = true;
+    if (s->precision == SWB_F64) return SWB_OK;  // the cell kernels start from the fields anyway
     set_fresh_kernel<<<1, 1, 0, s->stream>>>(s->a.ctl);
     swb::count_launches(1);
     CUDA_TRY(&s->err, cudaGetLastError());
-    s->host_fresh = true;
-    s->fields_current = true;
     return SWB_OK;
 }
 
@@ -613,6 +630,12 @@ bool persist_default(const swb_state *s) {
 // captured sequence is steady and the graph can be replayed at any time.
 cudaError_t launch_sequence(swb_state *s, int n) {
     cudaError_t e = cudaSuccess;
+    if (s->precision == SWB_F64) {
+        for (int k = 0; k < n && e == cudaSuccess; ++k) e = swb::launch_cell_step(s->a, s->x, k, s->stream);
+        StepArgs c = s->a;
+        c.meas_mask = 0;  // the cell kernels have reduced every iteration's measures
+        return e == cudaSuccess ? swb::launch_advance(c, n, s->stream) : e;
+    }
     for (int k = 0; k < n && e == cudaSuccess; ++k)
         e = swb::launch_fused_step(s->precision, s->a, k, !(s->host_fresh && k == 0), s->stream);
     if (e == cudaSuccess) e = swb::launch_advance(s->a, n, s->stream);
@@ -767,8 +790,11 @@ int autotune_geometry(swb_state *s, long long &left) {
 int fused_steps(swb_state *s, long long nsteps) {
     long long left = nsteps;
     const long long steps0 = s->steps;
-    const bool tune_now = !s->tuned && s->autotune && nsteps >= kTuneMinSteps;
-    if (s->host_fresh && left > 0) {
+    // Float64 lattices have one form (the cell kernels), which keep the fields
+    // current and so have no first iteration of another kind
+    const bool cells = s->precision == SWB_F64;
+    const bool tune_now = !cells && !s->tuned && s->autotune && nsteps >= kTuneMinSteps;
+    if (!cells && s->host_fresh && left > 0) {
         // the first iteration after the fields were set, alone (see launch_sequence)
         CUDA_TRY(&s->err, launch_sequence(s, 1));
         s->steps += 1;
@@ -816,7 +842,7 @@ int fused_steps(swb_state *s, long long nsteps) {
     s->steps = steps0 + nsteps;
     if (nsteps > 0) {
         s->host_fresh = false;
-        s->fields_current = false;
+        s->fields_current = cells;
     }
     return SWB_OK;
 }
@@ -869,7 +895,8 @@ int swb_state_bytes(const swb_params *p, int precision, size_t *bytes) {
         b = align256((size_t)27 * N * 8) + 11 * align256((size_t)N * 8);
     } else if (precision == SWB_F64 || precision == SWB_F32 || precision == SWB_F16) {
         b = 2 * align256(fbuf_bytes(precision, pitch)) + 3 * align256((size_t)N * real_bytes(precision)) +
-            align256((size_t)2 * tiles * swb::kNPart * 8) + align256(sizeof(Control)) +
+            (precision == SWB_F64 ? align256(cell_bytes(*p)) : align256((size_t)2 * tiles * swb::kNPart * 8)) +
+            align256(sizeof(Control)) +
             align256(swb::kBarWords * sizeof(unsigned int));
     } else {
         return fail(nullptr, SWB_ERR_ARG, "unknown precision");
@@ -950,8 +977,23 @@ int swb_create(const swb_params *p, int precision, swb_state **out) {
         int gnt = 0, gh = 0;
         swb::default_geometry(p->Lx, p->Ly, precision, &gnt, &gh);
         swb::set_geometry(a, gnt, gh);
-        a.part_stride = (int)swb::max_tiles(p->Lx, p->Ly);
-        CREATE_TRY(s->alloc((void **)&a.partials, (size_t)2 * a.part_stride * swb::kNPart * 8));
+        if (precision == SWB_F64) {
+            swb::Cell64 &x = s->x;
+            CREATE_TRY(s->alloc((void **)&x.p, cell_bytes(*p)));
+            x.wave = x.p + N;
+            x.acc = (unsigned long long *)(x.wave + 2 * (size_t)p->Lx);
+            CREATE_TRY(cudaMemsetAsync(x.acc, 0, 2 * swb::kAcc64 * 8, s->stream));
+            x.f = {1.0, -0.0};
+            x.mu6 = 6.0 * p->mu;
+            x.delta6 = 6.0 * p->delta;
+            x.delta3sq = 3.0 * (p->delta * p->delta);
+            x.g56 = (5.0 / 6.0) * p->g;
+            x.g15 = 1.5 * p->g;
+            x.thr_key = threshold_key(a.hthresh);
+        } else {
+            a.part_stride = (int)swb::max_tiles(p->Lx, p->Ly);
+            CREATE_TRY(s->alloc((void **)&a.partials, (size_t)2 * a.part_stride * swb::kNPart * 8));
+        }
         CREATE_TRY(s->alloc((void **)&a.ctl, sizeof(Control)));
         CREATE_TRY(s->alloc((void **)&a.bar, swb::kBarWords * sizeof(unsigned int)));
         CREATE_TRY(cudaMemsetAsync(a.bar, 0, swb::kBarWords * sizeof(unsigned int), s->stream));
@@ -1293,6 +1335,7 @@ int swb_set_measures(swb_state *s, int mask, double hthresh) {
     if (s->a.meas_mask == mask && s->a.hthresh == hthresh) return SWB_OK;
     s->a.meas_mask = mask;
     s->a.hthresh = hthresh;
+    s->x.thr_key = threshold_key(hthresh);
     s->plain_meas_mask = mask;
     s->invalidate_graph();
     return SWB_OK;

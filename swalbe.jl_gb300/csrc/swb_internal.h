@@ -111,6 +111,35 @@ struct StepArgs {
     long long stop_at;
 };
 
+// Sums, differences and products as fused multiply-adds.  On GB300 a stream
+// of DFMA issues every 16.5 cycles per SM, a stream of DADD or DMUL every 19.1
+// (measured, 4 to 32 warps per SM).  x * 1 + y rounds once, like x + y, and
+// x * y - 0 once, like x * y, signs of zero included.  `one` and `nzero` (1
+// and -0) come from the kernel's arguments: written as constants the compiler
+// would turn the forms back into sums and products.
+struct Fma64 {
+    double one, nzero;
+    __device__ __forceinline__ double add(double a, double b) const { return __fma_rn(a, one, b); }
+    __device__ __forceinline__ double sub(double a, double b) const { return __fma_rn(-b, one, a); }
+    __device__ __forceinline__ double mul(double a, double b) const { return __fma_rn(a, b, nzero); }
+};
+
+// What the Float64 cell kernels need beside the step arguments.
+constexpr int kChunks = 5;                // integers a Float64 sum is split into
+constexpr int kSums64 = 3 * kChunks + 1;  // mass, area, cos-sum, wetted count
+constexpr int kLanes64 = 16;
+// accumulators of one iteration parity: sums, hmax and hmin keys, each in
+// kLanes64 lanes, then the Float64 sums of values the integers do not hold
+constexpr int kAcc64 = (kSums64 + 2) * kLanes64 + 4;
+struct Cell64 {
+    Fma64 f;
+    double *p;                // film pressure of the iteration
+    double *wave;             // θ wave: κ and cospi(θ) of each column
+    unsigned long long *acc;  // [2][kAcc64]
+    double mu6, delta6, delta3sq, g56, g15;  // constants in the reference's order
+    unsigned long long thr_key;              // order-preserving key of hthresh
+};
+
 // Offset of the moving θ field at iteration t (1-based): it has moved
 // k = (t - 1 - t0) / tmove times (move_substrate! runs at the end of every
 // tmove-th iteration, scripts/Moving_wettability_structs.jl:139-152), and
@@ -259,7 +288,8 @@ cudaError_t launch_batch_step(int precision, int nt, bool gen, bool steady_tau1,
                               const StepArgs *d_args, const TileRef *d_tiles, int ntiles,
                               int grid, int k, cudaStream_t st, bool rare = true);
 int batch_blocks_per_sm(int precision, int nt, bool wave = false);
-cudaError_t launch_fused_step_f64(const StepArgs &a, int k, cudaStream_t st);
+// Iteration k of a sequence of a single Float64 lattice (its cell kernels; counts them).
+cudaError_t launch_cell_step(const StepArgs &a, const Cell64 &x, int k, cudaStream_t st);
 cudaError_t launch_moments_f64(const StepArgs &a, cudaStream_t st);
 cudaError_t launch_fout_f64(const StepArgs &a, double *out, cudaStream_t st);
 cudaError_t launch_pressure_now_f64(const StepArgs &a, double *out, cudaStream_t st);

@@ -5,6 +5,7 @@
 // Contents: the fused step in Float64 (literal arithmetic), the plain
 // one-kernel-per-reference-op path, and the standalone measure reduction.
 #include "swb_step_impl.cuh"
+#include "swb_f64.cuh"
 
 namespace swb {
 
@@ -23,13 +24,315 @@ namespace swb {
         }                                          \
     } while (0)
 
-cudaError_t launch_fused_step_f64(const StepArgs &a, int k, cudaStream_t st) {
-    const int grid = step_grid(a, k);
+// One iteration of a single Float64 lattice is three kernels of one cell per
+// thread: the film pressure of the fields, forces and collision into the
+// post-collision populations, and the moments of those populations back into
+// the fields (so h and u are always those of the iteration that comes next).
+//
+// Why not the strips of the FP32 states: the step is bound by the Float64
+// units (a warp instruction per 64 cycles and SM quarter), so what counts is
+// the number of Float64 instructions per cell and an even share of them for
+// every SM quarter; memory and the extra launches hide behind them.  A
+// strip recomputes the moments and pressures of its halo and leaves lanes
+// idle where the lattice is no multiple of it; one cell per thread does
+// neither, and needs no barrier.  Against strips with the plain operations
+// (302 Float64 instructions per cell, now about 145): 600 iterations of a
+// 256² droplet 41.1 -> 16.0 ms, 60 of a 1000 x 1030 film 34.3 -> 17.1 ms (upload
+// and download included), 200 of a 56 x 40 film 9.5 -> 3.3 ms.
+constexpr int kCellNT = 128;
+
+namespace {
+
+struct Cell {
+    int i, j, im, ip, jm, jp;  // column, row, and the periodic neighbours
+};
+__device__ __forceinline__ Cell cell_at(int c, int Lx, int Ly) {
+    Cell g;
+    g.j = c / Lx;
+    g.i = c - g.j * Lx;
+    g.im = g.i == 0 ? Lx - 1 : g.i - 1;
+    g.ip = g.i == Lx - 1 ? 0 : g.i + 1;
+    g.jm = (g.j == 0 ? Ly - 1 : g.j - 1) * Lx;
+    g.jp = (g.j == Ly - 1 ? 0 : g.j + 1) * Lx;
+    g.j *= Lx;  // rows as offsets
+    return g;
+}
+
+// κ and cospi(θ) of every column for iteration step_base + k + 1 of the θ wave.
+__global__ void __launch_bounds__(kCellNT) cell_wave_kernel(const StepArgs a, const Cell64 x, int k) {
+    grid_dep_wait();
+    grid_dep_launch();
+    const int i = blockIdx.x * kCellNT + threadIdx.x;
+    if (i >= a.Lx) return;
+    const KapCos<double> w = wave_at<double>(a, i, a.ctl->step_base + k + 1);
+    x.wave[i] = w.kap;
+    x.wave[a.Lx + i] = w.cs;
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kCellNT) cell_pressure_kernel(const StepArgs a, const Cell64 x, int k) {
+    const int c = blockIdx.x * kCellNT + threadIdx.x;
+    const int cc = c < a.Lx * a.Ly ? c : 0;
+    const Cell g = cell_at(cc, a.Lx, a.Ly);
+    grid_dep_wait();
+    grid_dep_launch();
+    if (c != cc) return;
+    const double *h = reinterpret_cast<const double *>(a.hF);
+    double kap = a.kap;
+    if (MODE == THETA_WAVE) kap = x.wave[g.i];
+    if (MODE == THETA_FIELD) {
+        int sx, sy;
+        substrate_shift(a, a.ctl->step_base + k + 1, &sx, &sy);
+        const int fi = g.i - sx < 0 ? g.i - sx + a.Lx : g.i - sx;
+        const int fj = g.j - sy * a.Lx < 0 ? g.j + (a.Ly - sy) * a.Lx : g.j - sy * a.Lx;
+        kap = reinterpret_cast<const double *>(a.kapF)[fj + fi];
+    }
+    x.p[c] = pressure64(x.f, h[c], h[g.j + g.im], h[g.jm + g.i], h[g.j + g.ip], h[g.jp + g.i],
+                        h[g.jm + g.im], h[g.jm + g.ip], h[g.jp + g.ip], h[g.jp + g.im], kap, a.gamma,
+                        a.hmin, a.hcrit, a.n, a.m);
+}
+
+// The measures of an iteration's height: every warp adds its cells' values
+// as integers (chunks64: exact, in any order), the block its warps', and one
+// atomic per value adds the block's to lane blockIdx % kLanes64.
+__device__ __forceinline__ void cell_measures(const StepArgs &a, const Cell64 &x, int par, bool in,
+                                              double h, double area, double cs, bool wet) {
+    __shared__ uint32_t sh[kCellNT / 32][kSums64 + 4];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const bool with_area = a.meas_mask & SWB_MEAS_AREA;
+    unsigned long long *acc = x.acc + (size_t)par * kAcc64;
+    double *big = reinterpret_cast<double *>(acc + kSums64 * kLanes64 + 2 * kLanes64);
+    uint32_t ch[kChunks];
+    auto add = [&](double v, bool on, int at) {
+#pragma unroll
+        for (int q = 0; q < kChunks; ++q) ch[q] = 0;
+        if (on && !chunks64(v, ch)) {
+#pragma unroll
+            for (int q = 0; q < kChunks; ++q) ch[q] = 0;
+            atomicAdd(big + at, v);
+        }
+#pragma unroll
+        for (int q = 0; q < kChunks; ++q) {
+            const uint32_t s = __reduce_add_sync(0xffffffffu, ch[q]);
+            if (lane == 0) sh[w][at * kChunks + q] = s;
+        }
+    };
+    add(h, in, 0);
+    if (with_area) {
+        add(area, wet, 1);
+        add(cs, wet, 2);
+    }
+    const uint32_t nwet = __popc(__ballot_sync(0xffffffffu, wet));
+    const unsigned long long o = in && h == h ? order64(h) : 0ull, o2 = o ? ~o : 0ull;
+    const uint32_t xh = __reduce_max_sync(0xffffffffu, (uint32_t)(o >> 32));
+    const uint32_t xl = __reduce_max_sync(0xffffffffu, (uint32_t)(o >> 32) == xh ? (uint32_t)o : 0u);
+    const uint32_t nh = __reduce_max_sync(0xffffffffu, (uint32_t)(o2 >> 32));
+    const uint32_t nl = __reduce_max_sync(0xffffffffu, (uint32_t)(o2 >> 32) == nh ? (uint32_t)o2 : 0u);
+    if (lane == 0) {
+        sh[w][kSums64 - 1] = nwet;
+        sh[w][kSums64] = xl;
+        sh[w][kSums64 + 1] = xh;
+        sh[w][kSums64 + 2] = nl;
+        sh[w][kSums64 + 3] = nh;
+    }
+    __syncthreads();
+    const int t = threadIdx.x, l = blockIdx.x % kLanes64;
+    if (t < kSums64) {
+        if (t >= kChunks && t < 3 * kChunks && !with_area) return;
+        const bool top = t < 3 * kChunks && t % kChunks == kChunks - 1;  // the signed chunk
+        long long s = 0;
+#pragma unroll
+        for (int q = 0; q < kCellNT / 32; ++q) s += top ? (long long)(int32_t)sh[q][t] : (long long)sh[q][t];
+        atomicAdd(acc + t * kLanes64 + l, (unsigned long long)s);
+    } else if (t >= 32 && t < 34) {
+        const int q0 = kSums64 + 2 * (t - 32);
+        unsigned long long m = 0;
+#pragma unroll
+        for (int q = 0; q < kCellNT / 32; ++q)
+            m = max(m, (unsigned long long)sh[q][q0 + 1] << 32 | sh[q][q0]);
+        atomicMax(acc + (kSums64 + t - 32) * kLanes64 + l, m);
+    }
+}
+
+// Reads, clears and sums the accumulators of iteration s and writes its
+// record: one block, beside the moments of the same iteration.
+__device__ void cell_reduce(const StepArgs &a, const Cell64 &x, long long s) {
+    __shared__ long long sum[kSums64];
+    __shared__ unsigned long long mx[2];
+    unsigned long long *acc = x.acc + (size_t)(s & 1) * kAcc64;
+    double *big = reinterpret_cast<double *>(acc + kSums64 * kLanes64 + 2 * kLanes64);
+    const int lane = threadIdx.x & (kLanes64 - 1), grp = threadIdx.x / kLanes64;
+    constexpr int G = kCellNT / kLanes64;  // fields handled at a time
+    static_assert(kLanes64 == 16 && (kSums64 + 2) % 2 == 0, "half-warp reductions");
+#pragma unroll
+    for (int f0 = 0; f0 < kSums64 + 2; f0 += G) {
+        const int f = f0 + grp;
+        const bool on = f < kSums64 + 2;
+        unsigned long long v = on ? __ldcg(acc + f * kLanes64 + lane) : 0ull;
+        if (on) acc[f * kLanes64 + lane] = 0ull;
+#pragma unroll
+        for (int o = kLanes64 / 2; o; o >>= 1) {
+            const unsigned long long w = __shfl_down_sync(0xffffffffu, v, o, kLanes64);
+            v = f < kSums64 ? v + w : max(v, w);
+        }
+        if (on && lane == 0) {
+            if (f < kSums64)
+                sum[f] = (long long)v;
+            else
+                mx[f - kSums64] = v;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double v[3];
+        for (int q = 0; q < 3; ++q) {
+            v[q] = value64(sum + q * kChunks);
+            const double b = __ldcg(big + q);
+            if (b != 0.0) {
+                v[q] += b;
+                big[q] = 0.0;
+            }
+        }
+        finish_step(a, s, v[0], (double)sum[kSums64 - 1], mx[0] ? unorder64(mx[0]) : -INFINITY,
+                    mx[1] ? unorder64(~mx[1]) : INFINITY, v[1], v[2]);
+    }
+}
+
+// Forces, equilibrium and collision (slippage!, h∇p!, the force sum,
+// thermal!, inclination!, equilibrium!, BGKandStream!'s collision).
+template <bool TAU1, bool G0, bool GEN>
+__global__ void __launch_bounds__(kCellNT) cell_collide_kernel(const StepArgs a, const Cell64 x, int k) {
+    const int c = blockIdx.x * kCellNT + threadIdx.x, N = a.Lx * a.Ly;
+    const int cc = c < N ? c : 0;
+    const Cell g = cell_at(cc, a.Lx, a.Ly);
+    // the sequence's step_base was written before the pressure kernel began
+    const long long done = __ldcg(&a.ctl->step_base) + k, tt = done + 1;
+    const int pitch = (int)a.pitch;
+    void *dst = (done & 1) ? a.fa : a.fb;
+    grid_dep_wait();
+    grid_dep_launch();
+    const bool in = c == cc;
+    double h = 0.0, area = 0.0, cs = 0.0;
+    bool wet = false;
+    if (in) {
+        const Fma64 &f = x.f;
+        h = reinterpret_cast<const double *>(a.hF)[c];
+        const double ux = reinterpret_cast<const double *>(a.uxF)[c];
+        const double uy = reinterpret_cast<const double *>(a.uyF)[c];
+        const double *p = x.p;
+        double gx, gy, sx, sy;
+        grad64(f, p[g.j + g.im], p[g.jm + g.i], p[g.j + g.ip], p[g.jp + g.i], p[g.jm + g.im],
+               p[g.jm + g.ip], p[g.jp + g.ip], p[g.jp + g.im], gx, gy);
+        slippage64(f, h, ux, uy, x.mu6, x.delta6, x.delta3sq, sx, sy);
+        double Fx = f.sub(-f.mul(h, gx), sx), Fy = f.sub(-f.mul(h, gy), sy);
+        if (GEN && a.thermal) {  // Fx .= -h∇px .- slipx .- kbtx (scripts/Rivulet_stability.jl:123)
+            double kx, ky;
+            thermal_force<true, double>(a.seed, (long long)c, tt, a.k6, h, a.delta, &kx, &ky);
+            Fx = Fx - kx;
+            Fy = Fy - ky;
+        }
+        if (GEN && a.incl) {  // inclination! (src/forcing.jl:364-365)
+            const double fac = a.incl_loop_time
+                                   ? 0.5 + 0.5 * tanh((double)(tt - a.incl_tstart) / (double)a.incl_tsmooth)
+                                   : a.incl_fixed;
+            Fx = Fx + (h * a.ax) * fac;
+            Fy = Fy + (h * a.ay) * fac;
+        }
+        double fe[9], fq[9];
+        if (!TAU1)
+            pull9<StoreF64>((done & 1) ? a.fb : a.fa, pitch, 1, g.i, g.j, g.im, g.ip, g.jm, g.jp, fq);
+        feq64<G0>(f, h, ux, uy, x.g56, x.g15, fe);
+        // sources of BGKandStream! (src/collide.jl:80-89)
+        const double S[4] = {f.mul(1.0 / 3.0, Fx), f.mul(1.0 / 3.0, Fy), f.mul(1.0 / 24.0, f.add(Fx, Fy)),
+                             f.mul(1.0 / 24.0, f.sub(Fy, Fx))};
+        constexpr int qp[4] = {1, 2, 5, 6}, qm[4] = {3, 4, 7, 8};
+        auto relax = [&](int q) {
+            return TAU1 ? fe[q] : f.add(f.mul(a.omeg, fq[q]), f.mul(a.invtau, fe[q]));
+        };
+        StoreF64::st(dst, pitch, 0, c, relax(0));
+#pragma unroll
+        for (int d = 0; d < 4; ++d) {
+            StoreF64::st(dst, pitch, qp[d], c, f.add(relax(qp[d]), S[d]));
+            StoreF64::st(dst, pitch, qm[d], c, f.sub(relax(qm[d]), S[d]));
+        }
+        if (!finite64(h)) a.ctl->nan_flag = 1;
+        // h > threshold, on the integer unit
+        wet = h == h && order64(h) > x.thr_key;
+        if ((a.meas_mask & SWB_MEAS_AREA) && wet) {
+            const double *hf = reinterpret_cast<const double *>(a.hF);
+            double gx2, gy2;
+            grad64(f, hf[g.j + g.im], hf[g.jm + g.i], hf[g.j + g.ip], hf[g.jp + g.i], hf[g.jm + g.im],
+                   hf[g.jm + g.ip], hf[g.jp + g.ip], hf[g.jp + g.im], gx2, gy2);
+            area = sqrt(gx2 * gx2 + gy2 * gy2 + 1.0);
+            if (GEN && a.theta_mode == THETA_FIELD) {
+                int tx, ty;
+                substrate_shift(a, tt, &tx, &ty);
+                const int fi = g.i - tx < 0 ? g.i - tx + a.Lx : g.i - tx;
+                const int fj = g.j - ty * a.Lx < 0 ? g.j + (a.Ly - ty) * a.Lx : g.j - ty * a.Lx;
+                cs = reinterpret_cast<const double *>(a.cosF)[fj + fi];
+            } else if (GEN && a.theta_mode == THETA_WAVE) {
+                cs = x.wave[a.Lx + g.i];
+            }
+        }
+    }
+    if (a.meas_mask) cell_measures(a, x, (int)(tt & 1), in, h, area, cs, wet);
+}
+
+// moments! of the populations the iteration wrote, pulled; the last block
+// reduces the iteration's measures.
+__global__ void __launch_bounds__(kCellNT) cell_moments_kernel(const StepArgs a, const Cell64 x, int k) {
+    const int c = blockIdx.x * kCellNT + threadIdx.x, N = a.Lx * a.Ly;
+    const int cc = c < N ? c : 0;
+    const Cell g = cell_at(cc, a.Lx, a.Ly);
+    const long long done = __ldcg(&a.ctl->step_base) + k;
+    const void *src = (done & 1) ? a.fa : a.fb;
+    grid_dep_wait();
+    grid_dep_launch();
+    if (a.meas_mask && blockIdx.x == gridDim.x - 1) {
+        cell_reduce(a, x, done + 1);
+        return;
+    }
+    if (c != cc) return;
+    double ft[9], h, jx, jy, ux, uy;
+    pull9<StoreF64>(src, (int)a.pitch, 1, g.i, g.j, g.im, g.ip, g.jm, g.jp, ft);
+    moments64(x.f, ft, h, jx, jy);
+    velocity64(x.f, h, jx, jy, ux, uy);
+    reinterpret_cast<double *>(a.hF)[c] = h;
+    reinterpret_cast<double *>(a.uxF)[c] = ux;
+    reinterpret_cast<double *>(a.uyF)[c] = uy;
+}
+
+}  // namespace
+
+cudaError_t launch_cell_step(const StepArgs &a, const Cell64 &x, int k, cudaStream_t st) {
+    const int grid = (int)(((long long)a.Lx * a.Ly + kCellNT - 1) / kCellNT);
     cudaError_t e = cudaSuccess;
-    if (step_general(a))
-        DISPATCH_NT(a.march_nt, e = launch_step(fused_step_kernel<StoreF64, NT, true>, grid, NT, st, a, k));
+    auto go = [&](auto kern, int blocks) {
+        if (e != cudaSuccess) return;
+        e = launch_step(kern, blocks, kCellNT, st, a, x, k);
+        count_launches(1);
+    };
+    if (a.theta_mode == THETA_WAVE) {
+        go(cell_wave_kernel, (a.Lx + kCellNT - 1) / kCellNT);
+        go(cell_pressure_kernel<THETA_WAVE>, grid);
+    } else if (a.theta_mode == THETA_FIELD) {
+        go(cell_pressure_kernel<THETA_FIELD>, grid);
+    } else {
+        go(cell_pressure_kernel<THETA_SCALAR>, grid);
+    }
+    const bool gen = step_general(a), g0 = a.g == 0.0;
+    auto collide = [&](auto t1, auto gz) {
+        constexpr bool T = decltype(t1)::value, G = decltype(gz)::value;
+        if (gen)
+            go(cell_collide_kernel<T, G, true>, grid);
+        else
+            go(cell_collide_kernel<T, G, false>, grid);
+    };
+    if (a.tau_is_one)
+        g0 ? collide(std::true_type{}, std::true_type{}) : collide(std::true_type{}, std::false_type{});
     else
-        DISPATCH_NT(a.march_nt, e = launch_step(fused_step_kernel<StoreF64, NT, false>, grid, NT, st, a, k));
+        g0 ? collide(std::false_type{}, std::true_type{}) : collide(std::false_type{}, std::false_type{});
+    go(cell_moments_kernel, grid + (a.meas_mask ? 1 : 0));
     return e;
 }
 
