@@ -1146,30 +1146,40 @@ int swb_set_theta_field(swb_state *s, const double *theta) {
     if (!s) return fail(nullptr, SWB_ERR_ARG, "state is NULL");
     if (!theta) return swb_set_theta(s, s->p.theta);
     const long long N = s->N;
-    std::vector<double> kap(N), cs(N);
-    for (long long i = 0; i < N; ++i) {
-        kap[i] = host_kappa(theta[i], s->p.n, s->p.m, s->p.hmin);
-        cs[i] = host_cospi(theta[i]);
-    }
     StepArgs &a = s->a;
+    void *dk = (void *)a.kapF, *dc = (void *)a.cosF;
     if (s->plain()) {
-        if (!s->plain_kapF) CUDA_TRY(&s->err, s->alloc((void **)&s->plain_kapF, (size_t)N * 8));
-        if (!s->plain_cosF) CUDA_TRY(&s->err, s->alloc((void **)&s->plain_cosF, (size_t)N * 8));
-        CUDA_TRY(&s->err, cudaMemcpyAsync(s->plain_kapF, kap.data(), N * 8, cudaMemcpyHostToDevice, s->stream));
-        CUDA_TRY(&s->err, cudaMemcpyAsync(s->plain_cosF, cs.data(), N * 8, cudaMemcpyHostToDevice, s->stream));
-        CUDA_TRY(&s->err, cudaStreamSynchronize(s->stream));
-    } else {
-        if (!a.kapF) {
-            void *k = nullptr, *c = nullptr;
-            CUDA_TRY(&s->err, s->alloc(&k, (size_t)N * s->rb()));
-            CUDA_TRY(&s->err, s->alloc(&c, (size_t)N * s->rb()));
-            a.kapF = k;
-            a.cosF = c;
+        dk = s->plain_kapF;
+        dc = s->plain_cosF;
+    }
+    if (!dk) CUDA_TRY(&s->err, s->alloc(&dk, (size_t)N * s->rb()));
+    if (!dc) CUDA_TRY(&s->err, s->alloc(&dc, (size_t)N * s->rb()));
+    int rc = ensure_tmp(s, (size_t)(N + 1) * 8);
+    if (rc) return rc;
+    int *hard = (int *)(s->dtmp + N), on_host = 0;
+    CUDA_TRY(&s->err, cudaMemcpyAsync(s->dtmp, theta, N * 8, cudaMemcpyHostToDevice, s->stream));
+    CUDA_TRY(&s->err, cudaMemsetAsync(hard, 0, sizeof(int), s->stream));
+    CUDA_TRY(&s->err, swb::launch_theta_field(s->dtmp, dk, dc, s->rb() == 8, N, s->p.n, s->p.m, s->p.hmin,
+                                              hard, s->stream));
+    CUDA_TRY(&s->err, cudaMemcpyAsync(&on_host, hard, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+    CUDA_TRY(&s->err, cudaStreamSynchronize(s->stream));
+    if (on_host) {
+        std::vector<double> kap(N), cs(N);
+        for (long long i = 0; i < N; ++i) {
+            kap[i] = host_kappa(theta[i], s->p.n, s->p.m, s->p.hmin);
+            cs[i] = host_cospi(theta[i]);
         }
-        int rc = upload_field(s, (void *)a.kapF, kap.data(), N);
+        rc = upload_field(s, dk, kap.data(), N);
         if (rc) return rc;
-        rc = upload_field(s, (void *)a.cosF, cs.data(), N);
+        rc = upload_field(s, dc, cs.data(), N);
         if (rc) return rc;
+    }
+    if (s->plain()) {
+        s->plain_kapF = (double *)dk;
+        s->plain_cosF = (double *)dc;
+    } else {
+        a.kapF = dk;
+        a.cosF = dc;
     }
     a.theta_mode = swb::THETA_FIELD;
     a.shift_tmove = 0;  // a new field starts at rest

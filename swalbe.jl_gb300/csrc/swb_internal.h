@@ -327,6 +327,11 @@ int pair_blocks_per_sm(int precision, int nt);
 int pair_rows(int Lx, int Ly, int precision, int nt);
 int batch_blocks_per_sm_f32(int precision, int nt, bool wave = false);
 
+// κ and cospi(θ) of a device θ field in the compute type; *hard (device) is
+// set where the host has to compute the field instead.
+cudaError_t launch_theta_field(const double *theta, void *kap, void *cs, bool is_double, long long N, int n,
+                               int m, double hmin, int *hard, cudaStream_t st);
+
 // plain FP64 per-op kernels (reference operation order)
 struct PlainState {
     int Lx, Ly;

@@ -97,3 +97,32 @@ def test_velocities_and_zeros():
         assert np.array_equal(x.height, lit.field("height"))
         assert np.array_equal(x.velx, lit.field("velx"))
         assert np.array_equal(x.vely, lit.field("vely"))
+
+
+@pytest.mark.parametrize("T,device", [(np.float64, "GB300"), (np.float64, "GB300-plain"), (np.float32, "GB300")])
+def test_theta_field_equals_scalar_theta(T, device):
+    """κ and cos θ of a field's cells are those of the same scalar θ: special
+    values, both sides of every reduction, and angles a hair from a right one."""
+    rng = np.random.default_rng(5)
+    th = [0.0, 0.25, 0.5, 0.75, 1.0, 1.5, 2.0, -0.3, 7.1, 1 / 9, 1e-200, 0.5 - 2.0 ** -54, 0.5 + 2.0 ** -50]
+    th += list(rng.uniform(0, 0.5, 60)) + list(rng.uniform(-3, 3, 20)) + list(0.25 + rng.uniform(-1e-9, 1e-9, 7))
+    for group in (th[:-12], th[:10] + th[14:]):
+        s = sw.SysConst(3, 1, sw.Taumucs())
+        one = sw.Sys(s, device, T=T)
+        want = []
+        for t in group:
+            one.set_theta(float(t))
+            want.append((probe(one, 3), one.measure_now().energy / 3))
+        s = sw.SysConst(len(group), 1, sw.Taumucs())
+        st = sw.Sys(s, device, T=T)
+        st.set_theta(np.array(group)[:, None])
+        got = probe(st, len(group))
+        assert np.array_equal(got, [w[0][0] for w in want])
+
+
+def probe(st, n):
+    """The film pressure of a flat film, which is κ times the same factor in every cell."""
+    st.height = np.full((n, 1), 0.07)
+    if st.precision == L.SWB_PLAIN64:
+        sw.api.check(sw.api.lib().swb_op_filmpressure(st.handle))
+    return st.pressure[:, 0]
