@@ -400,7 +400,7 @@ double swb_server_clock(swb_server *sv);
  * height 1, velocity 0.  SWB_F64 (the reference's arithmetic, bit for bit)
  * or SWB_F32.  rec_cap > 0 keeps the measures (mass, wetted count,
  * max/min) of the last rec_cap iterations of each lattice.  Every
- * swb1d_step runs all lattices together, one CTA each. */
+ * swb1d_step runs all lattices together. */
 typedef struct swb1d swb1d;
 #define SWB1D_FIELD_THETA 20 /* θ field (time_loop(sys, state, θ::Vector))          */
 #define SWB1D_FIELD_GAMMA 21 /* γ field and its ∇γ force (run_gamma, src/simulate.jl:518-556) */

@@ -11,162 +11,288 @@
 // in the reference's operation order (this unit is compiled with
 // --fmad=false), so Float64 results equal the oracle's bit for bit.
 //
-// 1D lattices are small, so a CTA owns a whole lattice and runs all the
-// iterations of a call in one launch: three phases per iteration (pressure,
-// collision with push streaming, moments) separated by __syncthreads; the
-// fields and populations stay in L2.  A batch of lattices is one CTA each.
-// No CTA waits for another.
+// A Float64 iteration of 128 cells takes an SM about 2 us (its Float64 units
+// finish a warp instruction every 16 cycles), whatever else is done, so the
+// cells of a lattice are spread over the SMs: a CTA of 128 threads, one cell
+// each, runs K iterations in registers and shared memory on its own cells and
+// a halo of 3 K cells on either side (an iteration reaches 3 cells: pressure,
+// force, streaming), recomputing the halo instead of exchanging it, and writes
+// its own cells to the other set of buffers.  (One CTA for a whole lattice
+// took 26.8 us per Float64 iteration of 1024 cells; this takes 3.3, with the
+// call's upload and reads.)  No CTA waits for another, and a
+// launch is paid once per K iterations.  Lattices of at most 128 cells fit one
+// CTA with no halo.
+#include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <cstring>
 #include <string>
 #include <vector>
 
+#include "swb_f64.cuh"
 #include "swb_lattice.h"
+#include "swb_step_impl.cuh"
 
 namespace swb {
+
+constexpr int kD1NT = 128;
 
 struct D1Args {
     int L;
     int n, m;
     double gamma, hmin, hcrit, delta, mu, g, kap, omeg, invtau;
-    void *fa, *fb;          // streamed populations (the reference's fout), 3 planes of L
-    void *h, *u, *p;        // fields (compute type)
-    const void *kapF;       // θ field: κ per cell (or null)
-    const void *gamF;       // γ field (or null)
-    const void *dgF;        // ∇γ of the γ field (or null)
-    Record *rec;            // per-iteration measures (ring of rec_cap, or null)
+    void *f[2], *h[2], *u[2];  // streamed populations (the reference's fout, 3 planes of L) and fields,
+                               // read from one set and written to the other by every launch
+    void *p;                   // pressure of the last iteration
+    const void *kapF;          // θ field: κ per cell (or null)
+    const void *gamF;          // γ field (or null)
+    const void *dgF;           // ∇γ of the γ field (or null)
+    Record *rec;               // per-iteration measures (ring of rec_cap, or null)
     int rec_cap;
-    long long *step;        // iterations done (device)
+    int chunk0, chunks;        // this lattice's entries of the chunk table
     int *nan_flag;
+};
+
+// The cells [x0, x0 + w) of a lattice, owned by one CTA.
+struct D1Chunk {
+    int lattice, x0, w;
+};
+
+// Measures of one warp's own cells at the start of one iteration.
+struct D1Part {
+    uint32_t mass[kChunks], wet;
+    unsigned long long kmax, kmin;
+    double big;
 };
 
 namespace {
 
-template <class R>
-__device__ __forceinline__ R pow_n(R x, int n) {  // power_broad (src/pressure.jl:363-369)
-    R t = R(1);
-    for (int i = 0; i < n; ++i) t *= x;
-    return t;
+// One cell's operations, Float64: rounded as the reference's, with products by
+// powers of two inside the sum that follows them (exact, short of subnormal
+// numbers).
+struct D1Ops64 {
+    Fma64 f;
+    __device__ __forceinline__ double quot(double a, double b) const {
+        bool hard = false;
+        const double q = quot64(a, b, recip64(b), f.nzero, hard);
+        return hard ? div64(a, b) : q;
+    }
+    __device__ __forceinline__ double pressure(const D1Args &a, double h, double hip, double him, double kap,
+                                               double gam) const {
+        double pn, pm;
+        powers64(f, quot(a.hmin, f.add(h, a.hcrit)), a.n, a.m, pn, pm);
+        const double p = f.mul(-gam, f.mul(kap, f.sub(pn, pm)));
+        return f.sub(p, f.mul(gam, f.add(__fma_rn(-2.0, h, hip), him)));
+    }
+    __device__ __forceinline__ double force(double h, double u, double pm, double pp, double mu6,
+                                            double delta6, double delta3sq) const {
+        const double den = f.add(__fma_rn(2.0, f.mul(h, h), f.mul(delta6, h)), delta3sq);
+        const double slip = quot(f.mul(f.mul(mu6, h), u), den);
+        return __fma_rn(0.5, f.mul(h, f.sub(pm, pp)), -slip);
+    }
+    __device__ __forceinline__ double sub(double a, double b) const { return f.sub(a, b); }
+    __device__ __forceinline__ void collide(double h, double u, double F, double g, double omeg, double invtau,
+                                            bool tau1, const double fo[3], double o[3]) const {
+        const double uu = f.mul(u, u);
+        double fe[3];
+        const double gh = g == 0.0 ? 0.0 : f.mul(0.25 * g, h);
+        fe[0] = f.mul(h, f.sub(g == 0.0 ? 1.0 : f.sub(1.0, f.mul(0.5 * g, h)), uu));
+        fe[1] = f.mul(h, __fma_rn(0.5, uu, __fma_rn(0.5, u, gh)));
+        fe[2] = f.mul(h, __fma_rn(0.5, uu, __fma_rn(-0.5, u, gh)));
+        if (!tau1)
+#pragma unroll
+            for (int q = 0; q < 3; ++q) fe[q] = f.add(f.mul(omeg, fo[q]), f.mul(invtau, fe[q]));
+        o[0] = fe[0];
+        o[1] = __fma_rn(0.5, F, fe[1]);
+        o[2] = __fma_rn(-0.5, F, fe[2]);
+    }
+    __device__ __forceinline__ void moments(const double o[3], double &h, double &u) const {
+        h = f.add(f.add(o[0], o[1]), o[2]);
+        u = quot(f.sub(o[1], o[2]), h);
+    }
+};
+
+// The same in FP32, operation by operation.
+struct D1Ops32 {
+    Fma64 f;  // (of Float64 states)
+    __device__ __forceinline__ static float pow_n(float x, int n) {  // power_broad (src/pressure.jl:363-369)
+        float t = 1.0f;
+        for (int i = 0; i < n; ++i) t *= x;
+        return t;
+    }
+    __device__ __forceinline__ float pressure(const D1Args &a, float h, float hip, float him, float kap,
+                                              float gam) const {
+        const float x = float(a.hmin) / (h + float(a.hcrit));
+        const float p = -gam * (kap * (pow_n(x, a.n) - pow_n(x, a.m)));
+        return p - gam * ((hip - 2.0f * h) + him);
+    }
+    __device__ __forceinline__ float force(float h, float u, float pm, float pp, float mu6, float delta6,
+                                           float delta3sq) const {
+        const float hgp = (h * -0.5f) * (pm - pp);
+        return -hgp - (mu6 * h * u) / ((2.0f * (h * h) + delta6 * h) + delta3sq);
+    }
+    __device__ __forceinline__ float sub(float a, float b) const { return a - b; }
+    __device__ __forceinline__ void collide(float h, float u, float F, float g, float omeg, float invtau, bool,
+                                            const float fo[3], float o[3]) const {
+        const float uu = u * u;
+        const float fe0 = h * ((1.0f - (0.5f * g) * h) - uu);
+        const float fe1 = h * (((0.25f * g) * h + 0.5f * u) + 0.5f * uu);
+        const float fe2 = h * (((0.25f * g) * h - 0.5f * u) + 0.5f * uu);
+        o[0] = omeg * fo[0] + invtau * fe0;
+        o[1] = omeg * fo[1] + invtau * fe1 + 0.5f * F;
+        o[2] = omeg * fo[2] + invtau * fe2 - 0.5f * F;
+    }
+    __device__ __forceinline__ void moments(const float o[3], float &h, float &u) const {
+        h = (o[0] + o[1]) + o[2];
+        u = (o[1] - o[2]) / h;
+    }
+};
+
+__device__ __forceinline__ bool finite(double v) { return finite64(v); }
+__device__ __forceinline__ bool finite(float v) { return isfinite(v); }
+
+// A warp's measures of its own cells' heights.
+__device__ __forceinline__ void d1_measure(D1Part *out, bool own, double h, bool wet) {
+    uint32_t c[kChunks] = {};
+    bool held = true;
+    if (own) held = chunks64(h, c);
+    const unsigned long long o = own && h == h ? order64(h) : 0ull, o2 = o ? ~o : 0ull;
+    D1Part p;
+    p.big = 0.0;
+    if (__any_sync(0xffffffffu, !held)) {
+        double b = held ? 0.0 : h;
+        if (!held)
+#pragma unroll
+            for (int q = 0; q < kChunks; ++q) c[q] = 0;
+        for (int k = 16; k; k >>= 1) b += __shfl_xor_sync(0xffffffffu, b, k);
+        p.big = b;
+    }
+#pragma unroll
+    for (int q = 0; q < kChunks; ++q) p.mass[q] = __reduce_add_sync(0xffffffffu, c[q]);
+    p.wet = __popc(__ballot_sync(0xffffffffu, own && wet));
+    const uint32_t xh = __reduce_max_sync(0xffffffffu, (uint32_t)(o >> 32));
+    const uint32_t xl = __reduce_max_sync(0xffffffffu, (uint32_t)(o >> 32) == xh ? (uint32_t)o : 0u);
+    const uint32_t nh = __reduce_max_sync(0xffffffffu, (uint32_t)(o2 >> 32));
+    const uint32_t nl = __reduce_max_sync(0xffffffffu, (uint32_t)(o2 >> 32) == nh ? (uint32_t)o2 : 0u);
+    p.kmax = (unsigned long long)xh << 32 | xl;
+    p.kmin = (unsigned long long)nh << 32 | nl;
+    if ((threadIdx.x & 31) == 0) *out = p;
 }
 
-template <class R>
-__device__ __forceinline__ void block_stats(R &mx, R &mn, double &sum, int &wet, R *sh,
-                                            double *shd, int *shi) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+// n iterations of the cells of chunk blockIdx.x, from the buffers `from` to the
+// others.  part: this launch's measures, [n][gridDim.x][kD1NT / 32] (or null).
+template <class R, class Ops>
+__global__ void __launch_bounds__(kD1NT) d1q3_run_kernel(const D1Args *__restrict__ args,
+                                                         const D1Chunk *__restrict__ table, const Ops op,
+                                                         int from, int n, D1Part *part) {
+    __shared__ D1Args a;
+    __shared__ R sh[kD1NT], sp[kD1NT], s1[kD1NT], s2[kD1NT];
+    const D1Chunk ck = table[blockIdx.x];
+    if (threadIdx.x == 0) a = args[ck.lattice];
+    __syncthreads();
+    grid_dep_wait();
+    grid_dep_launch();
+    const int t = threadIdx.x, L = a.L;
+    const bool whole = ck.w == L && L <= kD1NT;  // periodic within the CTA
+    const int halo = whole ? 0 : 3 * n, span = ck.w + 2 * halo;
+    const bool in = t < span, own = t >= halo && t < halo + ck.w;
+    int g = ck.x0 - halo + t;  // halo < L
+    g = g < 0 ? g + L : (g >= L ? g - L : g);
+    if (!in) g = 0;
+    // neighbours; at the ends of a span with halos their values do not matter
+    const int tm = t == 0 ? (whole ? span - 1 : 0) : t - 1;
+    const int tp = t >= span - 1 ? (whole ? 0 : span - 1) : t + 1;
+    const R mu6 = R(6) * R(a.mu), delta6 = R(6) * R(a.delta), delta3sq = R(3) * (R(a.delta) * R(a.delta));
+    const R omeg = R(a.omeg), invtau = R(a.invtau), grav = R(a.g);
+    const bool tau1 = a.omeg == 0.0 && a.invtau == 1.0;
+    const R kap = a.kapF ? reinterpret_cast<const R *>(a.kapF)[g] : R(a.kap);
+    const R gam = a.gamF ? reinterpret_cast<const R *>(a.gamF)[g] : R(a.gamma);
+    const R dg = a.dgF ? reinterpret_cast<const R *>(a.dgF)[g] : R(0);
+    const bool grad = a.dgF != nullptr, rec = part != nullptr && a.rec;
+    const R *ff = reinterpret_cast<const R *>(a.f[from]);
+    R h = reinterpret_cast<const R *>(a.h[from])[g], u = reinterpret_cast<const R *>(a.u[from])[g];
+    R fo[3] = {ff[g], ff[L + g], ff[2 * L + g]}, p = R(0);
+    int bad = 0;
+#pragma unroll 1
+    for (int k = 0; k < n; ++k) {
+        sh[t] = h;
+        __syncthreads();
+        if (rec)
+            d1_measure(part + ((size_t)k * gridDim.x + blockIdx.x) * (kD1NT / 32) + (t >> 5), own, (double)h,
+                       h > R(0.055));
+        if (in) {
+            p = op.pressure(a, h, sh[tm], sh[tp], kap, gam);
+            sp[t] = p;
+        }
+        __syncthreads();
+        R o[3];
+        if (in) {
+            R F = op.force(h, u, sp[tm], sp[tp], mu6, delta6, delta3sq);
+            if (grad) F = op.sub(F, dg);
+            op.collide(h, u, F, grav, omeg, invtau, tau1, fo, o);
+            s1[t] = o[1];
+            s2[t] = o[2];
+        }
+        __syncthreads();
+        if (in) {
+            fo[0] = o[0];
+            fo[1] = s1[tm];
+            fo[2] = s2[tp];
+            op.moments(fo, h, u);
+            if (own && !finite(h)) bad = 1;
+        }
+    }
+    if (own) {
+        R *fn = reinterpret_cast<R *>(a.f[from ^ 1]);
+        reinterpret_cast<R *>(a.h[from ^ 1])[g] = h;
+        reinterpret_cast<R *>(a.u[from ^ 1])[g] = u;
+        reinterpret_cast<R *>(a.p)[g] = p;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) fn[q * L + g] = fo[q];
+        if (bad) *a.nan_flag = 1;
+    }
+}
+
+// The records of n iterations after t0 from their warps' measures: one warp
+// per lattice (blockIdx.y) and iteration.
+__global__ void __launch_bounds__(128) d1q3_record_kernel(const D1Args *__restrict__ args,
+                                                          const D1Part *__restrict__ part, int nchunks,
+                                                          int n, long long t0) {
+    const D1Args &a = args[blockIdx.y];
+    const int k = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (k >= n || !a.rec || n - k > a.rec_cap) return;  // only the newest the ring holds
+    long long c[kChunks] = {};
+    unsigned long long mx = 0, mn = 0;
+    int wet = 0;
+    double big = 0.0;
+    const D1Part *pp = part + ((size_t)k * nchunks + a.chunk0) * (kD1NT / 32);
+    for (int i = lane; i < a.chunks * (kD1NT / 32); i += 32) {
+#pragma unroll
+        for (int q = 0; q < kChunks; ++q)
+            c[q] += q == kChunks - 1 ? (long long)(int32_t)pp[i].mass[q] : (long long)pp[i].mass[q];
+        wet += (int)pp[i].wet;
+        mx = max(mx, pp[i].kmax);
+        mn = max(mn, pp[i].kmin);
+        big += pp[i].big;
+    }
     for (int o = 16; o; o >>= 1) {
-        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+#pragma unroll
+        for (int q = 0; q < kChunks; ++q) c[q] += __shfl_xor_sync(0xffffffffu, c[q], o);
         wet += __shfl_xor_sync(0xffffffffu, wet, o);
+        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        mn = max(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        big += __shfl_xor_sync(0xffffffffu, big, o);
     }
     if (lane == 0) {
-        sh[w] = mx;
-        sh[32 + w] = mn;
-        shd[w] = sum;
-        shi[w] = wet;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int k = 1; k < nw; ++k) {
-            mx = fmax(mx, sh[k]);
-            mn = fmin(mn, sh[32 + k]);
-            sum += shd[k];
-            wet += shi[k];
-        }
-    }
-}
-
-// n iterations of lattice blockIdx.x.  rec_on: record the measures of the
-// height at the start of every iteration.
-template <class R>
-__global__ void __launch_bounds__(256) d1q3_run_kernel(const D1Args *__restrict__ args, int n) {
-    __shared__ R sh[64];
-    __shared__ double shd[32];
-    __shared__ int shi[32];
-    __shared__ D1Args a;
-    if (threadIdx.x == 0) a = args[blockIdx.x];
-    __syncthreads();
-    const int L = a.L, NT = blockDim.x;
-    R *h = reinterpret_cast<R *>(a.h), *u = reinterpret_cast<R *>(a.u), *p = reinterpret_cast<R *>(a.p);
-    const R *kapF = reinterpret_cast<const R *>(a.kapF);
-    const R *gamF = reinterpret_cast<const R *>(a.gamF);
-    const R *dgF = reinterpret_cast<const R *>(a.dgF);
-    const R gamma = R(a.gamma), hmin = R(a.hmin), hcrit = R(a.hcrit), g = R(a.g);
-    const R mu6 = R(6) * R(a.mu), delta6 = R(6) * R(a.delta), delta3sq = R(3) * (R(a.delta) * R(a.delta));
-    const R omeg = R(a.omeg), invtau = R(a.invtau), kap_s = R(a.kap);
-    const long long t0 = *a.step;
-    int bad = 0;
-    for (int k = 0; k < n; ++k) {
         const long long t = t0 + k + 1;
-        const R *fo = reinterpret_cast<const R *>(((t0 + k) & 1) ? a.fb : a.fa);
-        R *fn = reinterpret_cast<R *>(((t0 + k) & 1) ? a.fa : a.fb);
-        // A. film pressure (and the measures of the current height)
-        R mx = R(-INFINITY), mn = R(INFINITY);
-        double sum = 0.0;
-        int wet = 0;
-        for (int i = threadIdx.x; i < L; i += NT) {
-            const R hc = h[i], hip = h[i == 0 ? L - 1 : i - 1], him = h[i == L - 1 ? 0 : i + 1];
-            const R gi = gamF ? gamF[i] : gamma;
-            const R kap = kapF ? kapF[i] : kap_s;
-            const R x = hmin / (hc + hcrit);
-            R pi = -gi * (kap * (pow_n(x, a.n) - pow_n(x, a.m)));
-            pi = pi - gi * ((hip - R(2) * hc) + him);
-            p[i] = pi;
-            if (a.rec) {
-                mx = fmax(mx, hc);
-                mn = fmin(mn, hc);
-                sum += (double)hc;
-                wet += hc > R(0.055) ? 1 : 0;
-            }
-        }
-        if (a.rec) {
-            block_stats(mx, mn, sum, wet, sh, shd, shi);
-            if (threadIdx.x == 0) {
-                Record &r = a.rec[(t - 1) % a.rec_cap];
-                r.t = t;
-                r.mass = sum;
-                r.wetted = (double)wet;
-                r.hmax = (double)mx;
-                r.hmin = (double)mn;
-                r.area = 0.0;
-                r.cos_sum = 0.0;
-            }
-        }
-        __syncthreads();
-        // B. forces, equilibrium, collision; push streaming into fn
-        for (int i = threadIdx.x; i < L; i += NT) {
-            const int im = i == 0 ? L - 1 : i - 1, ip = i == L - 1 ? 0 : i + 1;
-            const R hc = h[i], uc = u[i];
-            const R hgp = (hc * R(-0.5)) * (p[im] - p[ip]);
-            const R slip = (mu6 * hc * uc) / ((R(2) * (hc * hc) + delta6 * hc) + delta3sq);
-            R F = -hgp - slip;
-            if (dgF) F = F - dgF[i];
-            const R uu = uc * uc;
-            const R fe0 = hc * ((R(1) - (R(0.5) * g) * hc) - uu);
-            const R fe1 = hc * (((R(0.25) * g) * hc + R(0.5) * uc) + R(0.5) * uu);
-            const R fe2 = hc * (((R(0.25) * g) * hc - R(0.5) * uc) + R(0.5) * uu);
-            const R o0 = omeg * fo[i] + invtau * fe0;
-            const R o1 = omeg * fo[L + i] + invtau * fe1 + R(0.5) * F;
-            const R o2 = omeg * fo[2 * L + i] + invtau * fe2 - R(0.5) * F;
-            fn[i] = o0;
-            fn[L + ip] = o1;
-            fn[2 * L + im] = o2;
-        }
-        __syncthreads();
-        // C. moments
-        for (int i = threadIdx.x; i < L; i += NT) {
-            const R f0 = fn[i], f1 = fn[L + i], f2 = fn[2 * L + i];
-            const R hh = (f0 + f1) + f2;
-            h[i] = hh;
-            u[i] = (f1 - f2) / hh;
-            if (!isfinite(hh)) bad = 1;
-        }
-        __syncthreads();
-    }
-    bad = __syncthreads_or(bad);
-    if (threadIdx.x == 0) {
-        *a.step = t0 + n;
-        if (bad) *a.nan_flag = 1;
+        Record &r = a.rec[(t - 1) % a.rec_cap];
+        r.t = t;
+        r.mass = value64(c) + big;
+        r.wetted = (double)wet;
+        r.hmax = mx ? unorder64(mx) : -INFINITY;
+        r.hmin = mn ? unorder64(~mn) : INFINITY;
+        r.area = 0.0;
+        r.cos_sum = 0.0;
     }
 }
 
@@ -199,9 +325,15 @@ struct swb1d {
     std::vector<D1Args> args;
     std::vector<char *> mem;  // one block per lattice
     D1Args *d_args = nullptr;
-    long long *d_steps = nullptr;
     int *d_flags = nullptr;
     int rec_cap = 0;
+    int cur = 0;               // buffers that hold the fields and populations
+    long long t = 0;           // iterations done
+    swb::D1Chunk *d_chunks = nullptr;
+    int nchunks = 0;
+    int per_launch = 0;        // iterations a launch may run
+    swb::D1Part *d_part = nullptr;
+    int part_steps = 0;        // iterations d_part holds
     bool args_dirty = true;
     cudaStream_t stream = nullptr;
     std::string err;
@@ -209,8 +341,9 @@ struct swb1d {
         if (stream) cudaStreamSynchronize(stream);
         for (char *q : mem) cudaFree(q);
         cudaFree(d_args);
-        cudaFree(d_steps);
         cudaFree(d_flags);
+        cudaFree(d_chunks);
+        cudaFree(d_part);
         if (stream) cudaStreamDestroy(stream);
     }
 };
@@ -224,11 +357,11 @@ struct swb1d {
     } while (0)
 
 namespace {
-// Bytes of one lattice's block: fa, fb (3L), h, u, p, κ, γ, ∇γ (L each) and
-// the measure ring.
+// Bytes of one lattice's block: two sets of populations (3L), h and u, then
+// p, κ, γ, ∇γ (L each) and the measure ring.
 size_t d1_bytes(int L, int rb, int rec_cap) {
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
-    return 2 * al((size_t)3 * L * rb) + 6 * al((size_t)L * rb) + al((size_t)rec_cap * sizeof(Record));
+    return 2 * al((size_t)3 * L * rb) + 8 * al((size_t)L * rb) + al((size_t)rec_cap * sizeof(Record));
 }
 
 int layout(swb1d *b, int i, char *base) {
@@ -236,10 +369,11 @@ int layout(swb1d *b, int i, char *base) {
     const int L = b->params[i].Lx, rb = b->rb;
     D1Args &a = b->args[i];
     size_t o = 0;
-    a.fa = base + o; o += al((size_t)3 * L * rb);
-    a.fb = base + o; o += al((size_t)3 * L * rb);
-    a.h = base + o; o += al((size_t)L * rb);
-    a.u = base + o; o += al((size_t)L * rb);
+    for (int k = 0; k < 2; ++k) {
+        a.f[k] = base + o; o += al((size_t)3 * L * rb);
+        a.h[k] = base + o; o += al((size_t)L * rb);
+        a.u[k] = base + o; o += al((size_t)L * rb);
+    }
     a.p = base + o; o += al((size_t)L * rb);
     o += 3 * al((size_t)L * rb);  // κ, γ, ∇γ: addressed through field_ptr
     a.rec = b->rec_cap ? reinterpret_cast<Record *>(base + o) : nullptr;
@@ -250,7 +384,7 @@ int layout(swb1d *b, int i, char *base) {
 char *field_ptr(swb1d *b, int i, int which) {  // 0 κ, 1 γ, 2 ∇γ (allocated slots)
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
     const int L = b->params[i].Lx, rb = b->rb;
-    return b->mem[i] + 2 * al((size_t)3 * L * rb) + (3 + which) * al((size_t)L * rb);
+    return b->mem[i] + 2 * al((size_t)3 * L * rb) + (5 + which) * al((size_t)L * rb);
 }
 
 int upload(swb1d *b, void *dst, const double *host, int L) {
@@ -284,6 +418,48 @@ __global__ void fill1(void *p, int L, int rb, double v) {
         else
             reinterpret_cast<float *>(p)[i] = (float)v;
     }
+}
+
+constexpr int kBurst = 4096;                  // iterations between records
+constexpr size_t kPartBytes = (size_t)64 << 20;  // of measures a burst keeps
+
+// Cuts the lattices into chunks of one CTA each and returns the iterations K
+// of a launch.  A launch of c CTAs per SM lasts about K max(1, c / r) t + t0:
+// Float64 t = 2 us and r = 1 (one CTA keeps an SM's Float64 units busy), FP32
+// t = 0.6 us and r = 8 (it leaves them idle), t0 = 2 us; larger K need more
+// CTAs, because 6 K of their 128 cells are halo.
+int split_lattices(swb1d *b, std::vector<swb::D1Chunk> &out) {
+    int sms = 1, dev = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 1;
+    const double t = b->rb == 8 ? 2.0 : 0.6, r = b->rb == 8 ? 1.0 : 8.0;
+    auto pieces = [&](int L, int K) {
+        const int w = swb::kD1NT - 6 * K;
+        return L <= swb::kD1NT ? 1 : (L + w - 1) / w;
+    };
+    int best = 1;
+    double cost = 1e300;
+    bool small = true;
+    for (const swb_params &p : b->params) small = small && p.Lx <= swb::kD1NT;
+    for (int K = 1; K <= 19; ++K) {
+        long long n = 0;
+        for (const swb_params &p : b->params) n += pieces(p.Lx, K);
+        const double c = std::max(1.0, std::ceil((double)n / sms) / r) * t + 2.0 / K;
+        if (c < cost) {
+            cost = c;
+            best = K;
+        }
+    }
+    for (int i = 0; i < b->count; ++i) {
+        const int L = b->params[i].Lx, k = pieces(L, best);
+        b->args[i].chunk0 = (int)out.size();
+        b->args[i].chunks = k;
+        for (int j = 0; j < k; ++j) {
+            const int x0 = (int)((long long)L * j / k), x1 = (int)((long long)L * (j + 1) / k);
+            out.push_back({i, x0, x1 - x0});
+        }
+    }
+    return small ? kBurst : best;  // without halos a launch may run any number of iterations
 }
 }  // namespace
 
@@ -327,9 +503,7 @@ int swb1d_create(const swb_params *params, int count, int precision, int rec_cap
         }                                                                                  \
     } while (0)
     C1_TRY(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
-    C1_TRY(cudaMalloc((void **)&b->d_steps, sizeof(long long) * count));
     C1_TRY(cudaMalloc((void **)&b->d_flags, sizeof(int) * count));
-    C1_TRY(cudaMemsetAsync(b->d_steps, 0, sizeof(long long) * count, b->stream));
     C1_TRY(cudaMemsetAsync(b->d_flags, 0, sizeof(int) * count, b->stream));
     C1_TRY(cudaMalloc((void **)&b->d_args, sizeof(D1Args) * count));
     for (int i = 0; i < count; ++i) {
@@ -354,12 +528,17 @@ int swb1d_create(const swb_params *params, int count, int precision, int rec_cap
         a.omeg = 1.0 - 1.0 / p.tau;
         a.invtau = 1.0 / p.tau;
         layout(b, i, m);
-        a.step = b->d_steps + i;
         a.nan_flag = b->d_flags + i;
-        fill1<<<(p.Lx + 255) / 256, 256, 0, b->stream>>>(a.h, p.Lx, b->rb, 1.0);  // height = 1
+        fill1<<<(p.Lx + 255) / 256, 256, 0, b->stream>>>(a.h[0], p.Lx, b->rb, 1.0);  // height = 1
         swb::count_launches(1);
         C1_TRY(cudaGetLastError());
     }
+    std::vector<swb::D1Chunk> chunks;
+    b->per_launch = split_lattices(b, chunks);
+    b->nchunks = (int)chunks.size();
+    C1_TRY(cudaMalloc((void **)&b->d_chunks, sizeof(swb::D1Chunk) * chunks.size()));
+    C1_TRY(cudaMemcpyAsync(b->d_chunks, chunks.data(), sizeof(swb::D1Chunk) * chunks.size(),
+                           cudaMemcpyHostToDevice, b->stream));
     C1_TRY(cudaStreamSynchronize(b->stream));
 #undef C1_TRY
     *out = b;
@@ -379,7 +558,7 @@ int swb1d_set_field(swb1d *b, int idx, int field, const double *host) {
         case SWB_FIELD_HEIGHT:
         case SWB_FIELD_VELX:
             if (!host) return d1fail(&b->err, SWB_ERR_ARG, "NULL field");
-            return upload(b, field == SWB_FIELD_HEIGHT ? a.h : a.u, host, L);
+            return upload(b, field == SWB_FIELD_HEIGHT ? a.h[b->cur] : a.u[b->cur], host, L);
         case SWB1D_FIELD_THETA: {
             if (!host) {
                 a.kapF = nullptr;
@@ -388,7 +567,10 @@ int swb1d_set_field(swb1d *b, int idx, int field, const double *host) {
             }
             std::vector<double> kap(L);
             const swb_params &p = b->params[idx];
-            for (int i = 0; i < L; ++i) kap[i] = swb::host_kappa_shared(host[i], p.n, p.m, p.hmin);
+            for (int i = 0; i < L; ++i)  // (fields are often constant over long stretches)
+                kap[i] = i > 0 && host[i] == host[i - 1]
+                             ? kap[i - 1]
+                             : swb::host_kappa_shared(host[i], p.n, p.m, p.hmin);
             char *dst = field_ptr(b, idx, 0);
             int rc = upload(b, dst, kap.data(), L);
             if (rc) return rc;
@@ -427,14 +609,11 @@ int swb1d_get_field(swb1d *b, int idx, int field, double *host) {
     if (!b || !host || idx < 0 || idx >= b->count)
         return d1fail(b ? &b->err : nullptr, SWB_ERR_ARG, "bad arguments");
     D1Args &a = b->args[idx];
-    long long t = 0;
-    D1_TRY(b, cudaMemcpyAsync(&t, a.step, sizeof(long long), cudaMemcpyDeviceToHost, b->stream));
-    D1_TRY(b, cudaStreamSynchronize(b->stream));
     switch (field) {
-        case SWB_FIELD_HEIGHT: return download(b, a.h, host, (size_t)a.L);
-        case SWB_FIELD_VELX: return download(b, a.u, host, (size_t)a.L);
+        case SWB_FIELD_HEIGHT: return download(b, a.h[b->cur], host, (size_t)a.L);
+        case SWB_FIELD_VELX: return download(b, a.u[b->cur], host, (size_t)a.L);
         case SWB_FIELD_PRESSURE: return download(b, a.p, host, (size_t)a.L);
-        case SWB_FIELD_FOUT: return download(b, (t & 1) ? a.fb : a.fa, host, (size_t)3 * a.L);
+        case SWB_FIELD_FOUT: return download(b, a.f[b->cur], host, (size_t)3 * a.L);
         default: return d1fail(&b->err, SWB_ERR_ARG, "1D fields: height, vel, pressure, fout");
     }
 }
@@ -446,15 +625,44 @@ int swb1d_step(swb1d *b, int64_t nsteps) {
                                   cudaMemcpyHostToDevice, b->stream));
         b->args_dirty = false;
     }
-    while (nsteps > 0) {  // launches of at most 4096 iterations
-        const int n = (int)(nsteps < 4096 ? nsteps : 4096);
-        if (b->rb == 8)
-            swb::d1q3_run_kernel<double><<<b->count, 256, 0, b->stream>>>(b->d_args, n);
-        else
-            swb::d1q3_run_kernel<float><<<b->count, 256, 0, b->stream>>>(b->d_args, n);
-        swb::count_launches(1);
-        D1_TRY(b, cudaGetLastError());
-        nsteps -= n;
+    // bursts of launches, then the burst's records
+    const size_t row = sizeof(swb::D1Part) * (swb::kD1NT / 32) * (size_t)b->nchunks;
+    while (nsteps > 0) {
+        int burst = (int)std::min<int64_t>(nsteps, kBurst);
+        if (b->rec_cap) {
+            burst = (int)std::min<size_t>((size_t)burst, std::max<size_t>(1, kPartBytes / row));
+            if (burst > b->part_steps) {
+                D1_TRY(b, cudaStreamSynchronize(b->stream));
+                cudaFree(b->d_part);
+                b->d_part = nullptr;
+                b->part_steps = 0;
+                D1_TRY(b, cudaMalloc((void **)&b->d_part, row * (size_t)burst));
+                b->part_steps = burst;
+            }
+        }
+        for (int done = 0; done < burst;) {
+            const int n = std::min(b->per_launch, burst - done);
+            swb::D1Part *part =
+                b->rec_cap ? b->d_part + (size_t)done * b->nchunks * (swb::kD1NT / 32) : nullptr;
+            const swb::Fma64 f{1.0, -0.0};
+            const cudaError_t e =
+                b->rb == 8 ? swb::launch_step(swb::d1q3_run_kernel<double, swb::D1Ops64>, b->nchunks, swb::kD1NT,
+                                              b->stream, b->d_args, b->d_chunks, swb::D1Ops64{f}, b->cur, n, part)
+                           : swb::launch_step(swb::d1q3_run_kernel<float, swb::D1Ops32>, b->nchunks, swb::kD1NT,
+                                              b->stream, b->d_args, b->d_chunks, swb::D1Ops32{f}, b->cur, n, part);
+            D1_TRY(b, e);
+            swb::count_launches(1);
+            b->cur ^= 1;
+            done += n;
+        }
+        if (b->rec_cap) {
+            swb::d1q3_record_kernel<<<dim3((unsigned)((burst + 3) / 4), (unsigned)b->count), 128, 0, b->stream>>>(
+                b->d_args, b->d_part, b->nchunks, burst, b->t);
+            swb::count_launches(1);
+            D1_TRY(b, cudaGetLastError());
+        }
+        b->t += burst;
+        nsteps -= burst;
     }
     return SWB_OK;
 }
@@ -475,8 +683,7 @@ int swb1d_get_measures(swb1d *b, int idx, swb_measure *out, int64_t cap, int64_t
     *count = 0;
     const D1Args &a = b->args[idx];
     if (!a.rec) return SWB_OK;
-    long long t = 0;
-    D1_TRY(b, cudaMemcpyAsync(&t, a.step, sizeof(long long), cudaMemcpyDeviceToHost, b->stream));
+    const long long t = b->t;
     D1_TRY(b, cudaStreamSynchronize(b->stream));
     long long n = t < a.rec_cap ? t : a.rec_cap;
     if (n > cap) n = cap;

@@ -56,7 +56,7 @@ __device__ __forceinline__ double quot64(double a, double b, double y, double nz
 }
 
 // The general division, out of line: its expansion stays out of the kernels.
-__device__ __noinline__ double div64(double a, double b) { return a / b; }
+static __device__ __noinline__ double div64(double a, double b) { return a / b; }
 
 // x^m and x^n by repeated multiplication as power_broad does
 // (src/pressure.jl:363-369); n > m >= 1, so x^m is met on the way to x^n.

@@ -5,7 +5,7 @@ Mirrors the reference's 1D API: ``SysConst_1D`` (src/initialize.jl:96-100),
 ``time_loop`` methods (src/simulate.jl:98-179), the 1D drivers and
 ``run_gamma`` (src/simulate.jl:247-560), ``two_droplets``
 (src/initialvalues.jl:277-323).  A state is one lattice of a ``Batch1D``;
-many 1D simulations run together, one CTA each, in one launch per call.
+many 1D simulations run together.
 """
 from __future__ import annotations
 
@@ -44,7 +44,7 @@ def _prec(T) -> int:
 
 
 class Batch1D:
-    """Many 1D lattices advanced together (one CTA per lattice)."""
+    """Many 1D lattices advanced together."""
 
     def __init__(self, systems: Sequence[SysConst_1D], T=np.float64, records: int = 0):
         self.systems = list(systems)
