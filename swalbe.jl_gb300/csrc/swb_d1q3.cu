@@ -70,45 +70,98 @@ namespace {
 // One cell's operations, Float64: rounded as the reference's, with products by
 // powers of two inside the sum that follows them (exact, short of subnormal
 // numbers).
+template <class O>
+struct D1Cell64 {
+    O o;
+    __device__ __forceinline__ double quot(double a, double b) { return o.quot(a, b, o.recip(b)); }
+    __device__ __forceinline__ double pressure(const D1Args &a, double h, double hip, double him, double kap,
+                                               double gam) {
+        double pn, pm;
+        powers64(o, quot(a.hmin, o.add(h, a.hcrit)), a.n, a.m, pn, pm);
+        const double p = o.mul(-gam, o.mul(kap, o.sub(pn, pm)));
+        return o.sub(p, o.mul(gam, o.add(o.twice_plus(-h, hip), him)));
+    }
+    __device__ __forceinline__ double force(double h, double u, double pm, double pp, double mu6,
+                                            double delta6, double delta3sq) {
+        const double den = o.add(o.twice_plus(o.muln(h, h), o.mul(delta6, h)), delta3sq);
+        const double slip = quot(o.mul(o.mul(mu6, h), u), den);
+        return __fma_rn(0.5, o.mul(h, o.sub(pm, pp)), -slip);
+    }
+    __device__ __forceinline__ double sub(double a, double b) { return o.sub(a, b); }
+    __device__ __forceinline__ void collide(double h, double u, double F, double g, double omeg, double invtau,
+                                            bool tau1, const double fo[3], double out[3]) {
+        const double uu = o.mul(u, u);
+        double fe[3];
+        const double gh = g == 0.0 ? 0.0 : o.muln(0.25 * g, h);
+        fe[0] = o.muln(h, o.sub(g == 0.0 ? 1.0 : o.sub(1.0, o.muln(0.5 * g, h)), uu));
+        fe[1] = o.mul(h, __fma_rn(0.5, uu, __fma_rn(0.5, u, gh)));
+        fe[2] = o.mul(h, __fma_rn(0.5, uu, __fma_rn(-0.5, u, gh)));
+        if (!tau1)
+#pragma unroll
+            for (int q = 0; q < 3; ++q) fe[q] = o.add(o.mul(omeg, fo[q]), o.mul(invtau, fe[q]));
+        out[0] = fe[0];
+        out[1] = __fma_rn(0.5, F, fe[1]);
+        out[2] = __fma_rn(-0.5, F, fe[2]);
+    }
+    __device__ __forceinline__ void moments(const double f[3], double &h, double &u) {
+        h = o.add(o.add(f[0], f[1]), f[2]);
+        u = quot(o.sub(f[1], f[2]), h);
+    }
+};
+// The three parts of an iteration with the integer unit's help, each computed
+// again out of line where that met a number it does not hold.
+__device__ __noinline__ double d1_pressure_again(const D1Args &a, double h, double hip, double him, double kap,
+                                                 double gam) {
+    return D1Cell64<Plain64>{}.pressure(a, h, hip, him, kap, gam);
+}
+__device__ __noinline__ double d1_force_again(double h, double u, double pm, double pp, double mu6,
+                                              double delta6, double delta3sq) {
+    return D1Cell64<Plain64>{}.force(h, u, pm, pp, mu6, delta6, delta3sq);
+}
+__device__ __noinline__ void d1_collide_again(double h, double u, double F, double g, double omeg,
+                                              double invtau, bool tau1, const double *fo, double *out) {
+    D1Cell64<Plain64>{}.collide(h, u, F, g, omeg, invtau, tau1, fo, out);
+}
+__device__ __noinline__ void d1_moments_again(const double *f, double *h, double *u) {
+    D1Cell64<Plain64>{}.moments(f, *h, *u);
+}
 struct D1Ops64 {
     Fma64 f;
-    __device__ __forceinline__ double quot(double a, double b) const {
-        bool hard = false;
-        const double q = quot64(a, b, recip64(b), f.nzero, hard);
-        return hard ? div64(a, b) : q;
-    }
     __device__ __forceinline__ double pressure(const D1Args &a, double h, double hip, double him, double kap,
                                                double gam) const {
-        double pn, pm;
-        powers64(f, quot(a.hmin, f.add(h, a.hcrit)), a.n, a.m, pn, pm);
-        const double p = f.mul(-gam, f.mul(kap, f.sub(pn, pm)));
-        return f.sub(p, f.mul(gam, f.add(__fma_rn(-2.0, h, hip), him)));
+        D1Cell64<Fast64> c{Fast64(f)};
+        const double p = c.pressure(a, h, hip, him, kap, gam);
+        return c.o.bad ? d1_pressure_again(a, h, hip, him, kap, gam) : p;
     }
     __device__ __forceinline__ double force(double h, double u, double pm, double pp, double mu6,
                                             double delta6, double delta3sq) const {
-        const double den = f.add(__fma_rn(2.0, f.mul(h, h), f.mul(delta6, h)), delta3sq);
-        const double slip = quot(f.mul(f.mul(mu6, h), u), den);
-        return __fma_rn(0.5, f.mul(h, f.sub(pm, pp)), -slip);
+        D1Cell64<Fast64> c{Fast64(f)};
+        const double F = c.force(h, u, pm, pp, mu6, delta6, delta3sq);
+        return c.o.bad ? d1_force_again(h, u, pm, pp, mu6, delta6, delta3sq) : F;
     }
     __device__ __forceinline__ double sub(double a, double b) const { return f.sub(a, b); }
     __device__ __forceinline__ void collide(double h, double u, double F, double g, double omeg, double invtau,
-                                            bool tau1, const double fo[3], double o[3]) const {
-        const double uu = f.mul(u, u);
-        double fe[3];
-        const double gh = g == 0.0 ? 0.0 : f.mul(0.25 * g, h);
-        fe[0] = f.mul(h, f.sub(g == 0.0 ? 1.0 : f.sub(1.0, f.mul(0.5 * g, h)), uu));
-        fe[1] = f.mul(h, __fma_rn(0.5, uu, __fma_rn(0.5, u, gh)));
-        fe[2] = f.mul(h, __fma_rn(0.5, uu, __fma_rn(-0.5, u, gh)));
-        if (!tau1)
+                                            bool tau1, const double fo[3], double out[3]) const {
+        D1Cell64<Fast64> c{Fast64(f)};
+        c.collide(h, u, F, g, omeg, invtau, tau1, fo, out);
+        if (c.o.bad) {
+            const double in[3] = {fo[0], fo[1], fo[2]};
+            double again[3];
+            d1_collide_again(h, u, F, g, omeg, invtau, tau1, in, again);
 #pragma unroll
-            for (int q = 0; q < 3; ++q) fe[q] = f.add(f.mul(omeg, fo[q]), f.mul(invtau, fe[q]));
-        o[0] = fe[0];
-        o[1] = __fma_rn(0.5, F, fe[1]);
-        o[2] = __fma_rn(-0.5, F, fe[2]);
+            for (int q = 0; q < 3; ++q) out[q] = again[q];
+        }
     }
-    __device__ __forceinline__ void moments(const double o[3], double &h, double &u) const {
-        h = f.add(f.add(o[0], o[1]), o[2]);
-        u = quot(f.sub(o[1], o[2]), h);
+    __device__ __forceinline__ void moments(const double fo[3], double &h, double &u) const {
+        D1Cell64<Fast64> c{Fast64(f)};
+        c.moments(fo, h, u);
+        if (c.o.bad) {
+            const double in[3] = {fo[0], fo[1], fo[2]};
+            double ha, ua;
+            d1_moments_again(in, &ha, &ua);
+            h = ha;
+            u = ua;
+        }
     }
 };
 

@@ -2,9 +2,12 @@
 //
 // Every operation rounds as the reference's does, so results equal the
 // oracle bit for bit; what changes is the unit that computes it.  GB300 has
-// one Float64 result per 64 FP32 ones (a warp instruction every 64 cycles on
-// each SM quarter), so Float64 kernels are bound by their count of Float64
-// instructions, and 30 integer instructions are cheaper than one division.
+// one Float64 result per 64 FP32 ones: a Float64 warp instruction occupies its
+// SM quarter's unit for 64 cycles or more, in which the quarter can issue some
+// forty integer instructions.  So about half of a cell's operations, the
+// products and the quotients, are computed with integers while the Float64
+// unit does the sums (Fast64).  Measured: products alone 15 cycles per SM and
+// warp, sums alone 16.5 to 19, one of each 19 together.
 #pragma once
 #include "swb_internal.h"
 
@@ -24,19 +27,55 @@ __device__ __forceinline__ double recip64(double b) {
     return __fma_rn(y, __fma_rn(e, e, e), y);
 }
 
+// a b rounded to nearest, of normal numbers or (ZERO) zeros, in integers: the
+// 106-bit product of the significands, its upper 62 or 63 bits with a sticky
+// last bit, rounded half to even at bit 10.  Sets `bad` where an operand or
+// the result is neither: the caller then computes the cell again (Plain64).
+__device__ __forceinline__ bool zero64(double v) { return ((hi64(v) & 0x7fffffffu) | lo64(v)) == 0; }
+template <bool ZERO>
+__device__ __forceinline__ double mul64(double a, double b, bool &bad) {
+    const uint32_t ah = hi64(a), bh = hi64(b);
+    // significands with their leading ones at bits 63 and 62
+    const uint32_t Ah = __funnelshift_l(lo64(a), (ah & 0xfffff) | 0x100000, 11), Al = lo64(a) << 11;
+    const uint32_t Bh = __funnelshift_l(lo64(b), (bh & 0xfffff) | 0x100000, 10), Bl = lo64(b) << 10;
+    const uint64_t p0 = (uint64_t)Al * Bl;
+    const uint64_t p1 = (uint64_t)Ah * Bl + (p0 >> 32);
+    const uint64_t p2 = (uint64_t)Al * Bh + (uint32_t)p1;
+    const uint64_t p = (uint64_t)Ah * Bh + (p1 >> 32) + (p2 >> 32);
+    const uint32_t sticky = (uint32_t)p0 | (uint32_t)p2;
+    uint32_t h = (uint32_t)(p >> 32), l = (uint32_t)p;
+    const uint32_t ea = (ah >> 20) & 0x7ff, eb = (bh >> 20) & 0x7ff;
+    uint32_t e = ea + eb - 1024;  // biased exponent less one
+    if (h & 0x40000000u) {
+        e += 1;
+    } else {
+        h = __funnelshift_l(l, h, 1);
+        l <<= 1;
+    }
+    l |= sticky ? 1u : 0u;
+    const uint64_t r = ((uint64_t)h << 32 | l) + (0x1ff + ((l >> 10) & 1));
+    uint32_t rl = __funnelshift_r((uint32_t)r, (uint32_t)(r >> 32), 10);
+    uint32_t rh = (uint32_t)(r >> 42) + (e << 20);  // the leading one adds the one e lacks
+    const bool zero = ZERO && (zero64(a) || zero64(b));
+    const bool off = (ea - 1u >= 2046u) | (eb - 1u >= 2046u) | (e >= 2045u);
+    if (zero) rl = rh = 0;
+    bad |= ZERO ? (off && !(zero && ea != 2047 && eb != 2047)) : off;
+    return __hiloint2double((int)(rh | ((ah ^ bh) & 0x80000000u)), (int)rl);
+}
+
 // a / b rounded to nearest from y = recip64(b): q = a y is within two ulp, and
 // the integer remainder R = A 2^s - B Q of the 53-bit significands (exact
 // modulo 2^64, and |R| < 2^56) says by how many ulp q is off, because q is
 // the nearest iff 2 |R| < B (a quotient of doubles is never half-way between
-// two doubles).  One Float64 instruction instead of about nine.  Sets `hard`
+// two doubles).  One Float64 instruction instead of about nine.  Sets `bad`
 // where that does not hold: exponents near the ends of the range, a q whose
-// neighbours may lie across a power of two, zero or non-finite b; the caller
-// then divides.  A zero a is exact as it is.
-__device__ __forceinline__ double quot64(double a, double b, double y, double nzero, bool &hard) {
+// neighbours across a power of two are spaced differently, zero or non-finite
+// b.  A zero a is exact as it is.
+__device__ __forceinline__ double quot64(double a, double b, double y, double nzero, bool &bad) {
     const double q = __fma_rn(a, y, nzero);
     const uint32_t ah = hi64(a), al = lo64(a), bh = hi64(b), bl = lo64(b), qh = hi64(q), ql = lo64(q);
     const uint32_t ea = (ah >> 20) & 0x7ff, eb = (bh >> 20) & 0x7ff, eq = (qh >> 20) & 0x7ff;
-    const bool zero = ((ah << 1) | al) == 0;
+    const bool zero = zero64(a);
     const uint32_t Bh = (bh & 0xfffff) | 0x100000, Qh = (qh & 0xfffff) | 0x100000;
     // s is 52 or 53, so the low word of A 2^s is zero and its high word is
     // A's low word shifted by s - 32
@@ -48,133 +87,164 @@ __device__ __forceinline__ double quot64(double a, double b, double y, double nz
     const int64_t T = 2 * (R < 0 ? -R : R);
     int k = (T > B ? 1 : 0) + (T > 3 * B ? 1 : 0);
     if (R < 0) k = -k;
-    const bool edge = (Qh == 0x1fffffu) | ((Qh == 0x100000u) & (ql < 4u));
+    // q at the bottom of a binade with a smaller quotient (the doubles below lie
+    // closer), or carried two steps from the last of one (those above do not)
+    const bool edge = ((Qh == 0x100000u) & (ql < 4u) & (R < 0)) | ((Qh == 0x1fffffu) & (ql == ~0u) & (k == 2));
     const bool range = (ea - 64u < 1919u) & (eq - 64u < 1919u);
-    hard |= (eb - 64u >= 1919u) | (!zero & (edge | !range));
+    bad |= (eb - 64u >= 1919u) | (!zero & (edge | !range));
     if (zero) k = 0;
     return __longlong_as_double(__double_as_longlong(q) + k);
 }
 
-// The general division, out of line: its expansion stays out of the kernels.
-static __device__ __noinline__ double div64(double a, double b) { return a / b; }
+// The operations of a cell.  mul: operands that may be zero; muln: operands
+// that are not (a zero is then computed again); twice_plus: 2 a + b, rounded
+// once either way because 2 a is exact.
+struct Fast64 {
+    Fma64 f;
+    bool bad;
+    __device__ __forceinline__ explicit Fast64(const Fma64 &g) : f(g.in_registers()), bad(false) {}
+    __device__ __forceinline__ double add(double a, double b) const { return f.add(a, b); }
+    __device__ __forceinline__ double sub(double a, double b) const { return f.sub(a, b); }
+    __device__ __forceinline__ double mul(double a, double b) { return mul64<true>(a, b, bad); }
+    __device__ __forceinline__ double muln(double a, double b) { return mul64<false>(a, b, bad); }
+    __device__ __forceinline__ double twice_plus(double a, double b) const { return __fma_rn(2.0, a, b); }
+    __device__ __forceinline__ double recip(double b) const { return recip64(b); }
+    __device__ __forceinline__ double quot(double a, double b, double y) {
+        return quot64(a, b, y, f.nzero, bad);
+    }
+};
+struct Plain64 {
+    __device__ __forceinline__ double add(double a, double b) const { return a + b; }
+    __device__ __forceinline__ double sub(double a, double b) const { return a - b; }
+    __device__ __forceinline__ double mul(double a, double b) const { return a * b; }
+    __device__ __forceinline__ double muln(double a, double b) const { return a * b; }
+    __device__ __forceinline__ double twice_plus(double a, double b) const { return 2.0 * a + b; }
+    __device__ __forceinline__ double recip(double) const { return 0.0; }
+    __device__ __forceinline__ double quot(double a, double b, double) const { return a / b; }
+};
 
 // x^m and x^n by repeated multiplication as power_broad does
 // (src/pressure.jl:363-369); n > m >= 1, so x^m is met on the way to x^n.
 // 1 * x is x.
-__device__ __forceinline__ void powers64(const Fma64 &f, double x, int n, int m, double &pn, double &pm) {
+template <class O>
+__device__ __forceinline__ void powers64(O &o, double x, int n, int m, double &pn, double &pm) {
     if (n == 9 && m == 3) {
-        const double x2 = f.mul(x, x);
-        pm = f.mul(x2, x);
+        const double x2 = o.muln(x, x);
+        pm = o.muln(x2, x);
         double t = pm;
 #pragma unroll
-        for (int i = 3; i < 9; ++i) t = f.mul(t, x);
+        for (int i = 3; i < 9; ++i) t = o.muln(t, x);
         pn = t;
     } else {
         double t = x;
         pm = x;
+#pragma unroll 1
         for (int i = 1; i < n; ++i) {
-            t = f.mul(t, x);
+            t = o.muln(t, x);
             if (i == m - 1) pm = t;
         }
         pn = t;
     }
 }
 
-// moments! (src/moments.jl:43-51), left to right.
-__device__ __forceinline__ void moments64(const Fma64 &f, const double p[9], double &h, double &jx,
-                                          double &jy) {
+// moments! (src/moments.jl:43-51), left to right: h and the momenta.
+template <class O>
+__device__ __forceinline__ void moments64(O &o, const double p[9], double &h, double &jx, double &jy) {
     // 0 + f0: f0, with -0 made +0
     double s = (hi64(p[0]) == 0x80000000u && lo64(p[0]) == 0u) ? 0.0 : p[0];
 #pragma unroll
-    for (int q = 1; q < 9; ++q) s = f.add(s, p[q]);
+    for (int q = 1; q < 9; ++q) s = o.add(s, p[q]);
     h = s;
-    jx = f.add(f.sub(f.sub(f.add(f.sub(p[1], p[3]), p[5]), p[6]), p[7]), p[8]);
-    jy = f.sub(f.sub(f.add(f.add(f.sub(p[2], p[4]), p[5]), p[6]), p[7]), p[8]);
+    jx = o.add(o.sub(o.sub(o.add(o.sub(p[1], p[3]), p[5]), p[6]), p[7]), p[8]);
+    jy = o.sub(o.sub(o.add(o.add(o.sub(p[2], p[4]), p[5]), p[6]), p[7]), p[8]);
 }
 
-// u = j / h.
-__device__ __forceinline__ void velocity64(const Fma64 &f, double h, double jx, double jy, double &ux,
-                                           double &uy) {
-    const double y = recip64(h);
-    bool hard = false;
-    ux = quot64(jx, h, y, f.nzero, hard);
-    uy = quot64(jy, h, y, f.nzero, hard);
-    if (hard) {
-        ux = div64(jx, h);
-        uy = div64(jy, h);
-    }
-}
+// The neighbours of a cell, named as in the reference: ip = v[i-1, j],
+// jp = v[i, j-1], im = v[i+1, j], jm = v[i, j+1], ...
+struct Near64 {
+    double ip, jp, im, jm, ipjp, imjp, imjm, ipjm;
+};
 
-// filmpressure! of one cell (src/pressure.jl:141-153); names as in pressure_cell.
-__device__ __forceinline__ double pressure64(const Fma64 &f, double h, double ip, double jp, double im,
-                                             double jm, double ipjp, double imjp, double imjm,
-                                             double ipjm, double kap, double gamma, double hmin,
-                                             double hcrit, int n, int m) {
-    const double d = f.add(h, hcrit);
-    bool hard = false;
-    double x = quot64(hmin, d, recip64(d), f.nzero, hard);
-    if (hard) x = div64(hmin, d);
+// filmpressure! of one cell (src/pressure.jl:141-153).
+template <class O>
+__device__ __forceinline__ double pressure64(O &o, double h, const Near64 &v, double kap, double gamma,
+                                             double hmin, double hcrit, int n, int m) {
+    const double d = o.add(h, hcrit);
+    const double x = o.quot(hmin, d, o.recip(d));
     double pn, pm;
-    powers64(f, x, n, m, pn, pm);
-    const double p = f.mul(-gamma, f.mul(kap, f.sub(pn, pm)));
-    const double near = f.mul(2.0 / 3.0, f.add(f.add(f.add(jp, ip), im), jm));
-    const double diag = f.mul(1.0 / 6.0, f.add(f.add(f.add(ipjp, imjp), imjm), ipjm));
-    const double lap = f.sub(f.add(near, diag), f.mul(10.0 / 3.0, h));
-    return f.sub(p, f.mul(gamma, lap));
+    powers64(o, x, n, m, pn, pm);
+    const double p = o.mul(-gamma, o.mul(kap, o.sub(pn, pm)));
+    const double near = o.muln(2.0 / 3.0, o.add(o.add(o.add(v.jp, v.ip), v.im), v.jm));
+    const double diag = o.muln(1.0 / 6.0, o.add(o.add(o.add(v.ipjp, v.imjp), v.imjm), v.ipjm));
+    const double lap = o.sub(o.add(near, diag), o.muln(10.0 / 3.0, h));
+    return o.sub(p, o.mul(gamma, lap));
 }
 
 // Gradient stencil of h∇p! (src/forcing.jl:181-184).
-__device__ __forceinline__ void grad64(const Fma64 &f, double ip, double jp, double im, double jm,
-                                       double ipjp, double imjp, double imjm, double ipjm, double &gx,
-                                       double &gy) {
-    gx = f.sub(f.mul(-1.0 / 3.0, f.sub(ip, im)),
-               f.mul(1.0 / 12.0, f.add(f.sub(f.sub(ipjp, imjp), imjm), ipjm)));
-    gy = f.sub(f.mul(-1.0 / 3.0, f.sub(jp, jm)),
-               f.mul(1.0 / 12.0, f.sub(f.sub(f.add(ipjp, imjp), imjm), ipjm)));
+template <class O>
+__device__ __forceinline__ void grad64(O &o, const Near64 &v, double &gx, double &gy) {
+    gx = o.sub(o.mul(-1.0 / 3.0, o.sub(v.ip, v.im)),
+               o.mul(1.0 / 12.0, o.add(o.sub(o.sub(v.ipjp, v.imjp), v.imjm), v.ipjm)));
+    gy = o.sub(o.mul(-1.0 / 3.0, o.sub(v.jp, v.jm)),
+               o.mul(1.0 / 12.0, o.sub(o.sub(o.add(v.ipjp, v.imjp), v.imjm), v.ipjm)));
 }
 
-// slippage! (src/forcing.jl:43-44): (6 μ h u) / (2 h^2 + 6 δ h + 3 δ^2).
-// 2 (h h) is exact, so it joins the sum in one rounding.
-__device__ __forceinline__ void slippage64(const Fma64 &f, double h, double ux, double uy, double mu6,
-                                           double delta6, double delta3sq, double &sx, double &sy) {
-    const double den = f.add(__fma_rn(2.0, f.mul(h, h), f.mul(delta6, h)), delta3sq);
-    const double mh = f.mul(mu6, h), nx = f.mul(mh, ux), ny = f.mul(mh, uy), y = recip64(den);
-    bool hard = false;
-    sx = quot64(nx, den, y, f.nzero, hard);
-    sy = quot64(ny, den, y, f.nzero, hard);
-    if (hard) {
-        sx = div64(nx, den);
-        sy = div64(ny, den);
+// -h ∇p - slip (src/simulate.jl:18-19) with slippage!'s
+// (6 μ h u) / (2 h^2 + 6 δ h + 3 δ^2) (src/forcing.jl:43-44).
+template <class O>
+__device__ __forceinline__ void force64(O &o, double h, double ux, double uy, double gx, double gy,
+                                        double mu6, double delta6, double delta3sq, double &Fx, double &Fy) {
+    const double den = o.add(o.twice_plus(o.muln(h, h), o.mul(delta6, h)), delta3sq);
+    const double mh = o.mul(mu6, h), y = o.recip(den);
+    const double sx = o.quot(o.mul(mh, ux), den, y), sy = o.quot(o.mul(mh, uy), den, y);
+    Fx = o.sub(-o.mul(h, gx), sx);
+    Fy = o.sub(-o.mul(h, gy), sy);
+}
+
+// equilibrium! (src/equilibrium.jl:67-114); g56 = 5/6 g, g15 = 1.5 g.  G0: no
+// gravity.  Then g h is an exact zero for a finite h and 0 + x is x (a zero x
+// only ever meets another term), so those operations are left out; a
+// non-finite h gives NaN in every population either way.
+template <bool G0, class O>
+__device__ __forceinline__ void feq64(O &o, double h, double ux, double uy, double g56, double g15,
+                                      double fe[9]) {
+    const double hh = (!G0 || finite64(h)) ? h : __longlong_as_double(0x7ff8000000000000LL);
+    const double xx = o.mul(ux, ux), yy = o.mul(uy, uy), vsq = o.add(xx, yy);
+    const double v15 = o.mul(1.5, vsq), v23 = o.mul(2.0 / 3.0, vsq);
+    if (G0)
+        fe[0] = o.muln(hh, o.sub(1.0, v23));
+    else
+        fe[0] = o.muln(hh, o.sub(o.sub(1.0, o.mul(g56, hh)), v23));
+    const double gh = G0 ? 0.0 : o.mul(g15, hh);
+    const double s = o.add(ux, uy), d = o.sub(uy, ux);
+    const double cu[4] = {ux, uy, s, d};
+    const double cc[4] = {xx, yy, o.mul(s, s), o.mul(d, d)};
+    // q and its opposite: 1/3, 2/4, 5/7, 6/8
+    constexpr int qp[4] = {1, 2, 5, 6}, qm[4] = {3, 4, 7, 8};
+    const double w[2] = {o.muln(1.0 / 9.0, hh), o.muln(1.0 / 36.0, hh)};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const double c3 = o.mul(3.0, cu[k]), c45 = o.mul(4.5, cc[k]);
+        const double tp = G0 ? c3 : o.add(gh, c3), tm = G0 ? -c3 : o.sub(gh, c3);
+        fe[qp[k]] = o.mul(w[k / 2], o.sub(o.add(tp, c45), v15));
+        fe[qm[k]] = o.mul(w[k / 2], o.sub(o.add(tm, c45), v15));
     }
 }
 
-// equilibrium! (src/equilibrium.jl:67-114); g56 = 5/6 g, g15 = 1.5 g.  G0: no gravity.  Then g h is an
-// exact zero for a finite h and 0 + x is x (a zero x only ever meets another
-// term), so those operations are left out; a non-finite h gives NaN in every
-// population either way.
-template <bool G0>
-__device__ __forceinline__ void feq64(const Fma64 &f, double h, double ux, double uy, double g56,
-                                      double g15, double fe[9]) {
-    const double hh = (!G0 || finite64(h)) ? h : __longlong_as_double(0x7ff8000000000000LL);
-    const double xx = f.mul(ux, ux), yy = f.mul(uy, uy), vsq = f.add(xx, yy);
-    const double v15 = f.mul(1.5, vsq), v23 = f.mul(2.0 / 3.0, vsq);
-    if (G0)
-        fe[0] = f.mul(hh, f.sub(1.0, v23));
-    else
-        fe[0] = f.mul(hh, f.sub(f.sub(1.0, f.mul(g56, hh)), v23));
-    const double gh = G0 ? 0.0 : f.mul(g15, hh);
-    const double s = f.add(ux, uy), d = f.sub(uy, ux);
-    const double cu[4] = {ux, uy, s, d};
-    const double cc[4] = {xx, yy, f.mul(s, s), f.mul(d, d)};
-    // q and its opposite: 1/3, 2/4, 5/7, 6/8
+// BGKandStream!'s collision (src/collide.jl:76-89): relaxation towards fe and
+// the sources of the force; fq (the streamed populations) only for τ != 1.
+template <bool TAU1, class O>
+__device__ __forceinline__ void relax64(O &o, const double fe[9], const double fq[9], double omeg,
+                                        double invtau, double Fx, double Fy, double out[9]) {
+    const double S[4] = {o.mul(1.0 / 3.0, Fx), o.mul(1.0 / 3.0, Fy), o.mul(1.0 / 24.0, o.add(Fx, Fy)),
+                         o.mul(1.0 / 24.0, o.sub(Fy, Fx))};
     constexpr int qp[4] = {1, 2, 5, 6}, qm[4] = {3, 4, 7, 8};
 #pragma unroll
+    for (int q = 0; q < 9; ++q) out[q] = TAU1 ? fe[q] : o.add(o.mul(omeg, fq[q]), o.mul(invtau, fe[q]));
+#pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const double w = f.mul(k < 2 ? 1.0 / 9.0 : 1.0 / 36.0, hh);
-        const double c3 = f.mul(3.0, cu[k]), c45 = f.mul(4.5, cc[k]);
-        const double tp = G0 ? c3 : f.add(gh, c3), tm = G0 ? -c3 : f.sub(gh, c3);
-        fe[qp[k]] = f.mul(w, f.sub(f.add(tp, c45), v15));
-        fe[qm[k]] = f.mul(w, f.sub(f.add(tm, c45), v15));
+        out[qp[k]] = o.add(out[qp[k]], S[k]);
+        out[qm[k]] = o.sub(out[qm[k]], S[k]);
     }
 }
 

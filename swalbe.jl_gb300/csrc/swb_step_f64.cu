@@ -36,9 +36,12 @@ namespace swb {
 // strip recomputes the moments and pressures of its halo and leaves lanes
 // idle where the lattice is no multiple of it; one cell per thread does
 // neither, and needs no barrier.  Against strips with the plain operations
-// (302 Float64 instructions per cell, now about 145): 600 iterations of a
-// 256² droplet 41.1 -> 16.0 ms, 60 of a 1000 x 1030 film 34.3 -> 17.1 ms (upload
-// and download included), 200 of a 56 x 40 film 9.5 -> 3.3 ms.
+// (302 Float64 instructions per cell; here 145, and with the products in
+// integers 94): 600 iterations of a 256² droplet 41.1 -> 16.0 -> 12.6 ms, 60 of a
+// 1000 x 1030 film 34.3 -> 17.1 -> 13.2 ms (upload and download included), 512²
+// 141 -> 77 -> 57 us per iteration.  A 56 x 40 film, one warp per SM quarter, is
+// bound by latency: 43.7 -> 10.7 -> 11.1 us.  (One kernel of 8 x 4 tiles with
+// recomputed halos: 9.4 there, but 12.4 at 128 x 96 and 104 at 512².)
 constexpr int kCellNT = 128;
 
 namespace {
@@ -58,6 +61,11 @@ __device__ __forceinline__ Cell cell_at(int c, int Lx, int Ly) {
     return g;
 }
 
+// Index into a θ field moved by (sx, sy), of column i and row offset j.
+__device__ __forceinline__ int field_at(const StepArgs &a, int i, int j, int sx, int sy) {
+    return (j - sy * a.Lx < 0 ? j + (a.Ly - sy) * a.Lx : j - sy * a.Lx) + (i - sx < 0 ? i - sx + a.Lx : i - sx);
+}
+
 // κ and cospi(θ) of every column for iteration step_base + k + 1 of the θ wave.
 __global__ void __launch_bounds__(kCellNT) cell_wave_kernel(const StepArgs a, const Cell64 x, int k) {
     grid_dep_wait();
@@ -67,6 +75,27 @@ __global__ void __launch_bounds__(kCellNT) cell_wave_kernel(const StepArgs a, co
     const KapCos<double> w = wave_at<double>(a, i, a.ctl->step_base + k + 1);
     x.wave[i] = w.kap;
     x.wave[a.Lx + i] = w.cs;
+}
+
+__device__ __forceinline__ Near64 near_cell(const double *v, const Cell &g) {
+    return {v[g.j + g.im],  v[g.jm + g.i],  v[g.j + g.ip],  v[g.jp + g.i],
+            v[g.jm + g.im], v[g.jm + g.ip], v[g.jp + g.ip], v[g.jp + g.im]};
+}
+
+// A cell whose integer arithmetic met a number it does not hold, again in
+// Float64 operations (out of line).
+__device__ __noinline__ double cell_pressure_again(double h, const Near64 &v, double kap, double gamma,
+                                                   double hmin, double hcrit, int n, int m) {
+    Plain64 o;
+    return pressure64(o, h, v, kap, gamma, hmin, hcrit, n, m);
+}
+__device__ __forceinline__ double cell_pressure(const StepArgs &a, const Cell64 &x, double h, const Near64 &v,
+                                                double kap) {
+    Fast64 o(x.f);
+    const double p = pressure64(o, h, v, kap, a.gamma, a.hmin, a.hcrit, a.n, a.m);
+    if (!o.bad) return p;
+    const Near64 w = v;
+    return cell_pressure_again(h, w, kap, a.gamma, a.hmin, a.hcrit, a.n, a.m);
 }
 
 template <int MODE>
@@ -83,21 +112,18 @@ __global__ void __launch_bounds__(kCellNT) cell_pressure_kernel(const StepArgs a
     if (MODE == THETA_FIELD) {
         int sx, sy;
         substrate_shift(a, a.ctl->step_base + k + 1, &sx, &sy);
-        const int fi = g.i - sx < 0 ? g.i - sx + a.Lx : g.i - sx;
-        const int fj = g.j - sy * a.Lx < 0 ? g.j + (a.Ly - sy) * a.Lx : g.j - sy * a.Lx;
-        kap = reinterpret_cast<const double *>(a.kapF)[fj + fi];
+        kap = reinterpret_cast<const double *>(a.kapF)[field_at(a, g.i, g.j, sx, sy)];
     }
-    x.p[c] = pressure64(x.f, h[c], h[g.j + g.im], h[g.jm + g.i], h[g.j + g.ip], h[g.jp + g.i],
-                        h[g.jm + g.im], h[g.jm + g.ip], h[g.jp + g.ip], h[g.jp + g.im], kap, a.gamma,
-                        a.hmin, a.hcrit, a.n, a.m);
+    x.p[c] = cell_pressure(a, x, h[c], near_cell(h, g), kap);
 }
 
 // The measures of an iteration's height: every warp adds its cells' values
 // as integers (chunks64: exact, in any order), the block its warps', and one
 // atomic per value adds the block's to lane blockIdx % kLanes64.
+template <int NT>
 __device__ __forceinline__ void cell_measures(const StepArgs &a, const Cell64 &x, int par, bool in,
                                               double h, double area, double cs, bool wet) {
-    __shared__ uint32_t sh[kCellNT / 32][kSums64 + 4];
+    __shared__ uint32_t sh[NT / 32][kSums64 + 4];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const bool with_area = a.meas_mask & SWB_MEAS_AREA;
     unsigned long long *acc = x.acc + (size_t)par * kAcc64;
@@ -142,27 +168,28 @@ __device__ __forceinline__ void cell_measures(const StepArgs &a, const Cell64 &x
         const bool top = t < 3 * kChunks && t % kChunks == kChunks - 1;  // the signed chunk
         long long s = 0;
 #pragma unroll
-        for (int q = 0; q < kCellNT / 32; ++q) s += top ? (long long)(int32_t)sh[q][t] : (long long)sh[q][t];
+        for (int q = 0; q < NT / 32; ++q) s += top ? (long long)(int32_t)sh[q][t] : (long long)sh[q][t];
         atomicAdd(acc + t * kLanes64 + l, (unsigned long long)s);
-    } else if (t >= 32 && t < 34) {
-        const int q0 = kSums64 + 2 * (t - 32);
+    } else if (t < kSums64 + 2) {
+        const int q0 = kSums64 + 2 * (t - kSums64);
         unsigned long long m = 0;
 #pragma unroll
-        for (int q = 0; q < kCellNT / 32; ++q)
+        for (int q = 0; q < NT / 32; ++q)
             m = max(m, (unsigned long long)sh[q][q0 + 1] << 32 | sh[q][q0]);
-        atomicMax(acc + (kSums64 + t - 32) * kLanes64 + l, m);
+        atomicMax(acc + t * kLanes64 + l, m);
     }
 }
 
 // Reads, clears and sums the accumulators of iteration s and writes its
-// record: one block, beside the moments of the same iteration.
+// record: one block, beside a later kernel.
+template <int NT>
 __device__ void cell_reduce(const StepArgs &a, const Cell64 &x, long long s) {
     __shared__ long long sum[kSums64];
     __shared__ unsigned long long mx[2];
     unsigned long long *acc = x.acc + (size_t)(s & 1) * kAcc64;
     double *big = reinterpret_cast<double *>(acc + kSums64 * kLanes64 + 2 * kLanes64);
     const int lane = threadIdx.x & (kLanes64 - 1), grp = threadIdx.x / kLanes64;
-    constexpr int G = kCellNT / kLanes64;  // fields handled at a time
+    constexpr int G = NT / kLanes64;  // fields handled at a time
     static_assert(kLanes64 == 16 && (kSums64 + 2) % 2 == 0, "half-warp reductions");
 #pragma unroll
     for (int f0 = 0; f0 < kSums64 + 2; f0 += G) {
@@ -198,16 +225,94 @@ __device__ void cell_reduce(const StepArgs &a, const Cell64 &x, long long s) {
     }
 }
 
-// Forces, equilibrium and collision (slippage!, h∇p!, the force sum,
-// thermal!, inclination!, equilibrium!, BGKandStream!'s collision).
+// Forces, equilibrium and collision of one cell (slippage!, h∇p!, the force
+// sum, thermal!, inclination!, equilibrium!, BGKandStream!'s collision).
+struct CollideIn {
+    double h, ux, uy;
+    Near64 p;
+    double kx, ky, ix, iy;  // thermal! and inclination! forces (GEN)
+    double fq[9];           // streamed populations (τ != 1)
+};
+template <bool TAU1, bool G0, bool GEN, class O>
+__device__ __forceinline__ void collide64(O &o, const StepArgs &a, const Cell64 &x, const CollideIn &v,
+                                          double out[9]) {
+    double gx, gy, Fx, Fy, fe[9];
+    grad64(o, v.p, gx, gy);
+    force64(o, v.h, v.ux, v.uy, gx, gy, x.mu6, x.delta6, x.delta3sq, Fx, Fy);
+    if (GEN && a.thermal) {  // Fx .= -h∇px .- slipx .- kbtx (scripts/Rivulet_stability.jl:123)
+        Fx = o.sub(Fx, v.kx);
+        Fy = o.sub(Fy, v.ky);
+    }
+    if (GEN && a.incl) {  // inclination! (src/forcing.jl:364-365)
+        Fx = o.add(Fx, v.ix);
+        Fy = o.add(Fy, v.iy);
+    }
+    feq64<G0>(o, v.h, v.ux, v.uy, x.g56, x.g15, fe);
+    relax64<TAU1>(o, fe, v.fq, a.omeg, a.invtau, Fx, Fy, out);
+}
 template <bool TAU1, bool G0, bool GEN>
-__global__ void __launch_bounds__(kCellNT) cell_collide_kernel(const StepArgs a, const Cell64 x, int k) {
+__device__ __noinline__ void cell_collide_again(const StepArgs &a, const Cell64 &x, const CollideIn &v,
+                                                double out[9]) {
+    Plain64 o;
+    collide64<TAU1, G0, GEN>(o, a, x, v, out);
+}
+
+// Collides cell c (its fields, pressures and streamed populations in v) in
+// iteration tt and stores the nine populations.
+template <bool TAU1, bool G0, bool GEN>
+__device__ __forceinline__ void cell_collide(const StepArgs &a, const Cell64 &x, CollideIn &v, int c,
+                                             long long tt, void *dst) {
+    if (GEN && a.thermal) thermal_force<true, double>(a.seed, (long long)c, tt, a.k6, v.h, a.delta, &v.kx, &v.ky);
+    if (GEN && a.incl) {
+        const double fac = a.incl_loop_time
+                               ? 0.5 + 0.5 * tanh((double)(tt - a.incl_tstart) / (double)a.incl_tsmooth)
+                               : a.incl_fixed;
+        v.ix = (v.h * a.ax) * fac;
+        v.iy = (v.h * a.ay) * fac;
+    }
+    double out[9];
+    Fast64 o(x.f);
+    collide64<TAU1, G0, GEN>(o, a, x, v, out);
+    if (o.bad) {
+        const CollideIn w = v;
+        double again[9];
+        cell_collide_again<TAU1, G0, GEN>(a, x, w, again);
+#pragma unroll
+        for (int q = 0; q < 9; ++q) out[q] = again[q];
+    }
+#pragma unroll
+    for (int q = 0; q < 9; ++q) StoreF64::st(dst, (int)a.pitch, q, c, out[q]);
+    if (!finite64(v.h)) a.ctl->nan_flag = 1;
+}
+
+// The surface element of a wetted cell and its cos θ.
+template <bool GEN>
+__device__ __forceinline__ void cell_area(const StepArgs &a, const Cell64 &x, const Near64 &h, int i, int j,
+                                          long long tt, double &area, double &cs) {
+    Plain64 o;
+    double gx, gy;
+    grad64(o, h, gx, gy);
+    area = sqrt(gx * gx + gy * gy + 1.0);
+    if (GEN && a.theta_mode == THETA_FIELD) {
+        int sx, sy;
+        substrate_shift(a, tt, &sx, &sy);
+        cs = reinterpret_cast<const double *>(a.cosF)[field_at(a, i, j, sx, sy)];
+    } else if (GEN && a.theta_mode == THETA_WAVE) {
+        cs = x.wave[a.Lx + i];
+    }
+}
+
+// Six blocks per SM (80 registers, 36 bytes of spill) instead of the four that
+// the compiler's 106 registers leave: 256² 24.9 -> 19.9 us per iteration, 301 x
+// 257 30.6 -> 20.8, 1000 x 1030 208 -> 195.
+template <bool TAU1, bool G0, bool GEN>
+__global__ void __launch_bounds__(kCellNT, 6) cell_collide_kernel(const __grid_constant__ StepArgs a,
+                                                               const __grid_constant__ Cell64 x, int k) {
     const int c = blockIdx.x * kCellNT + threadIdx.x, N = a.Lx * a.Ly;
     const int cc = c < N ? c : 0;
     const Cell g = cell_at(cc, a.Lx, a.Ly);
     // the sequence's step_base was written before the pressure kernel began
     const long long done = __ldcg(&a.ctl->step_base) + k, tt = done + 1;
-    const int pitch = (int)a.pitch;
     void *dst = (done & 1) ? a.fa : a.fb;
     grid_dep_wait();
     grid_dep_launch();
@@ -215,67 +320,38 @@ __global__ void __launch_bounds__(kCellNT) cell_collide_kernel(const StepArgs a,
     double h = 0.0, area = 0.0, cs = 0.0;
     bool wet = false;
     if (in) {
-        const Fma64 &f = x.f;
-        h = reinterpret_cast<const double *>(a.hF)[c];
-        const double ux = reinterpret_cast<const double *>(a.uxF)[c];
-        const double uy = reinterpret_cast<const double *>(a.uyF)[c];
-        const double *p = x.p;
-        double gx, gy, sx, sy;
-        grad64(f, p[g.j + g.im], p[g.jm + g.i], p[g.j + g.ip], p[g.jp + g.i], p[g.jm + g.im],
-               p[g.jm + g.ip], p[g.jp + g.ip], p[g.jp + g.im], gx, gy);
-        slippage64(f, h, ux, uy, x.mu6, x.delta6, x.delta3sq, sx, sy);
-        double Fx = f.sub(-f.mul(h, gx), sx), Fy = f.sub(-f.mul(h, gy), sy);
-        if (GEN && a.thermal) {  // Fx .= -h∇px .- slipx .- kbtx (scripts/Rivulet_stability.jl:123)
-            double kx, ky;
-            thermal_force<true, double>(a.seed, (long long)c, tt, a.k6, h, a.delta, &kx, &ky);
-            Fx = Fx - kx;
-            Fy = Fy - ky;
-        }
-        if (GEN && a.incl) {  // inclination! (src/forcing.jl:364-365)
-            const double fac = a.incl_loop_time
-                                   ? 0.5 + 0.5 * tanh((double)(tt - a.incl_tstart) / (double)a.incl_tsmooth)
-                                   : a.incl_fixed;
-            Fx = Fx + (h * a.ax) * fac;
-            Fy = Fy + (h * a.ay) * fac;
-        }
-        double fe[9], fq[9];
+        const double *hf = reinterpret_cast<const double *>(a.hF);
+        CollideIn v;
+        h = v.h = hf[c];
+        v.ux = reinterpret_cast<const double *>(a.uxF)[c];
+        v.uy = reinterpret_cast<const double *>(a.uyF)[c];
+        v.p = near_cell(x.p, g);
         if (!TAU1)
-            pull9<StoreF64>((done & 1) ? a.fb : a.fa, pitch, 1, g.i, g.j, g.im, g.ip, g.jm, g.jp, fq);
-        feq64<G0>(f, h, ux, uy, x.g56, x.g15, fe);
-        // sources of BGKandStream! (src/collide.jl:80-89)
-        const double S[4] = {f.mul(1.0 / 3.0, Fx), f.mul(1.0 / 3.0, Fy), f.mul(1.0 / 24.0, f.add(Fx, Fy)),
-                             f.mul(1.0 / 24.0, f.sub(Fy, Fx))};
-        constexpr int qp[4] = {1, 2, 5, 6}, qm[4] = {3, 4, 7, 8};
-        auto relax = [&](int q) {
-            return TAU1 ? fe[q] : f.add(f.mul(a.omeg, fq[q]), f.mul(a.invtau, fe[q]));
-        };
-        StoreF64::st(dst, pitch, 0, c, relax(0));
-#pragma unroll
-        for (int d = 0; d < 4; ++d) {
-            StoreF64::st(dst, pitch, qp[d], c, f.add(relax(qp[d]), S[d]));
-            StoreF64::st(dst, pitch, qm[d], c, f.sub(relax(qm[d]), S[d]));
-        }
-        if (!finite64(h)) a.ctl->nan_flag = 1;
-        // h > threshold, on the integer unit
-        wet = h == h && order64(h) > x.thr_key;
-        if ((a.meas_mask & SWB_MEAS_AREA) && wet) {
-            const double *hf = reinterpret_cast<const double *>(a.hF);
-            double gx2, gy2;
-            grad64(f, hf[g.j + g.im], hf[g.jm + g.i], hf[g.j + g.ip], hf[g.jp + g.i], hf[g.jm + g.im],
-                   hf[g.jm + g.ip], hf[g.jp + g.ip], hf[g.jp + g.im], gx2, gy2);
-            area = sqrt(gx2 * gx2 + gy2 * gy2 + 1.0);
-            if (GEN && a.theta_mode == THETA_FIELD) {
-                int tx, ty;
-                substrate_shift(a, tt, &tx, &ty);
-                const int fi = g.i - tx < 0 ? g.i - tx + a.Lx : g.i - tx;
-                const int fj = g.j - ty * a.Lx < 0 ? g.j + (a.Ly - ty) * a.Lx : g.j - ty * a.Lx;
-                cs = reinterpret_cast<const double *>(a.cosF)[fj + fi];
-            } else if (GEN && a.theta_mode == THETA_WAVE) {
-                cs = x.wave[a.Lx + g.i];
-            }
-        }
+            pull9<StoreF64>((done & 1) ? a.fb : a.fa, (int)a.pitch, 1, g.i, g.j, g.im, g.ip, g.jm, g.jp, v.fq);
+        cell_collide<TAU1, G0, GEN>(a, x, v, c, tt, dst);
+        wet = h == h && order64(h) > x.thr_key;  // h > threshold, on the integer unit
+        if ((a.meas_mask & SWB_MEAS_AREA) && wet) cell_area<GEN>(a, x, near_cell(hf, g), g.i, g.j, tt, area, cs);
     }
-    if (a.meas_mask) cell_measures(a, x, (int)(tt & 1), in, h, area, cs, wet);
+    if (a.meas_mask) cell_measures<kCellNT>(a, x, (int)(tt & 1), in, h, area, cs, wet);
+}
+
+// u = j / h of a cell whose quotients the integers do not hold.
+__device__ __noinline__ void cell_velocity_again(double h, double jx, double jy, double *ux, double *uy) {
+    *ux = jx / h;
+    *uy = jy / h;
+}
+__device__ __forceinline__ void cell_velocity(const Cell64 &x, double h, double jx, double jy, double &ux,
+                                              double &uy) {
+    Fast64 o(x.f);
+    const double y = o.recip(h);
+    ux = o.quot(jx, h, y);
+    uy = o.quot(jy, h, y);
+    if (o.bad) {
+        double vx, vy;
+        cell_velocity_again(h, jx, jy, &vx, &vy);
+        ux = vx;
+        uy = vy;
+    }
 }
 
 // moments! of the populations the iteration wrote, pulled; the last block
@@ -289,29 +365,42 @@ __global__ void __launch_bounds__(kCellNT) cell_moments_kernel(const StepArgs a,
     grid_dep_wait();
     grid_dep_launch();
     if (a.meas_mask && blockIdx.x == gridDim.x - 1) {
-        cell_reduce(a, x, done + 1);
+        cell_reduce<kCellNT>(a, x, done + 1);
         return;
     }
     if (c != cc) return;
     double ft[9], h, jx, jy, ux, uy;
     pull9<StoreF64>(src, (int)a.pitch, 1, g.i, g.j, g.im, g.ip, g.jm, g.jp, ft);
-    moments64(x.f, ft, h, jx, jy);
-    velocity64(x.f, h, jx, jy, ux, uy);
+    Fast64 o(x.f);
+    moments64(o, ft, h, jx, jy);
+    cell_velocity(x, h, jx, jy, ux, uy);
     reinterpret_cast<double *>(a.hF)[c] = h;
     reinterpret_cast<double *>(a.uxF)[c] = ux;
     reinterpret_cast<double *>(a.uyF)[c] = uy;
 }
 
+template <class F>
+void by_kind(const StepArgs &a, F f) {  // f(TAU1, G0, GEN)
+    const bool gen = step_general(a), g0 = a.g == 0.0;
+    using T = std::true_type;
+    using N = std::false_type;
+    auto go = [&](auto t, auto g) { gen ? f(t, g, T{}) : f(t, g, N{}); };
+    if (!a.tau_is_one)
+        go(N{}, N{});
+    else
+        g0 ? go(T{}, T{}) : go(T{}, N{});
+}
+
 }  // namespace
 
 cudaError_t launch_cell_step(const StepArgs &a, const Cell64 &x, int k, cudaStream_t st) {
-    const int grid = (int)(((long long)a.Lx * a.Ly + kCellNT - 1) / kCellNT);
     cudaError_t e = cudaSuccess;
     auto go = [&](auto kern, int blocks) {
         if (e != cudaSuccess) return;
         e = launch_step(kern, blocks, kCellNT, st, a, x, k);
         count_launches(1);
     };
+    const int grid = (int)(((long long)a.Lx * a.Ly + kCellNT - 1) / kCellNT);
     if (a.theta_mode == THETA_WAVE) {
         go(cell_wave_kernel, (a.Lx + kCellNT - 1) / kCellNT);
         go(cell_pressure_kernel<THETA_WAVE>, grid);
@@ -320,18 +409,9 @@ cudaError_t launch_cell_step(const StepArgs &a, const Cell64 &x, int k, cudaStre
     } else {
         go(cell_pressure_kernel<THETA_SCALAR>, grid);
     }
-    const bool gen = step_general(a), g0 = a.g == 0.0;
-    auto collide = [&](auto t1, auto gz) {
-        constexpr bool T = decltype(t1)::value, G = decltype(gz)::value;
-        if (gen)
-            go(cell_collide_kernel<T, G, true>, grid);
-        else
-            go(cell_collide_kernel<T, G, false>, grid);
-    };
-    if (a.tau_is_one)
-        g0 ? collide(std::true_type{}, std::true_type{}) : collide(std::true_type{}, std::false_type{});
-    else
-        g0 ? collide(std::false_type{}, std::true_type{}) : collide(std::false_type{}, std::false_type{});
+    by_kind(a, [&](auto t, auto g, auto gen) {
+        go(cell_collide_kernel<decltype(t)::value, decltype(g)::value, decltype(gen)::value>, grid);
+    });
     go(cell_moments_kernel, grid + (a.meas_mask ? 1 : 0));
     return e;
 }
