@@ -376,7 +376,7 @@ int swb_server_set_policy(swb_server *sv, int policy, int64_t max_resident_cells
 /* Strip geometry of the resident set.  nt = 0 (default): chosen whenever the
  * set changes (pair strips of 60 or 124 columns, whichever processes fewer
  * cells, when every lattice allows pair strips; one-column strips of 64
- * threads otherwise), each lattice's rows balanced up to `rows` (0: 64).
+ * threads otherwise), each lattice's rows balanced up to `rows` (0: chosen for the set, at most 64).
  * nt = -32 or -64: those pair strips whenever every lattice allows them,
  * rows balanced up to `rows` (>= 2).  Results do not depend on the
  * geometry. */

@@ -178,37 +178,59 @@ bool admit_device(swb_server *sv, Req *r) {
 // so the strip width is chosen for the set: 124 columns (64 threads) or 60
 // (32 threads), whichever processes fewer cells in all (60-column strips
 // waste less on the small lattices a shortest-job-first queue favours).
-// Rows are set per lattice to the balanced height of at most 64 rows that
-// covers it (a 64-row lattice is one strip, 100 rows two of 50).  Results
-// do not depend on the geometry.
+// Rows are set per lattice to the balanced height of at most `cap` rows that
+// covers it (a 64-row lattice is one strip, 100 rows two of 50), with the cap
+// (up to 64) chosen for the set as well: an iteration lasts at least as long as
+// one CTA's march over its tallest strip (iteration_us), so a set that does not
+// fill the GPU takes short strips although they recompute more.  Results do
+// not depend on the geometry.
 constexpr int kServePairRows = 64;
 int balanced_rows(int Ly, int cap) {
     const int strips = (Ly + cap - 1) / cap;
     return (Ly + strips - 1) / strips;
 }
-double padded_cells(const std::vector<Req *> &set, int nt, int cap) {
-    const int w = -2 * nt - 4;
-    double n = 0.0;
-    for (const Req *r : set) {
+// Estimated time of an iteration with strips of geometry nt and at most cap
+// rows: the march of the tallest strip at one row's latency, or the padded
+// cells at the full GPU's rate, whichever is longer.  The constants were
+// measured on GB300: a lone pair strip of 64 rows takes 49 us (0.7 us per
+// row), a full resident set runs 80 cells per ns; one-column strips 0.6 us and
+// 55; Float64 strips 10 us and 2.  (Eight lattices of 32k to 147k cells: 50 us
+// per iteration with 64 rows.)
+double iteration_us(const swb_server *sv, int nt, int cap) {
+    const bool f64 = sv->precision == SWB_F64;
+    const double row = nt < 0 ? 0.7 : (f64 ? 10.0 : 0.6), rate = nt < 0 ? 80e3 : (f64 ? 2e3 : 55e3);
+    const int w = nt < 0 ? -2 * nt - 4 : nt - 4;
+    double cells = 0.0;
+    int tallest = 0;
+    for (const Req *r : sv->active) {
         const int h = balanced_rows(r->p.Ly, cap);
-        n += (double)((r->p.Lx + w - 1) / w) * (w + 4) * (double)((r->p.Ly + h - 1) / h) * (h + 4);
+        tallest = std::max(tallest, h);
+        cells += (double)((r->p.Lx + w - 1) / w) * (w + 4) * (double)((r->p.Ly + h - 1) / h) * (h + 4);
     }
-    return n;
+    // (the small term lets fewer cells decide between equal marches)
+    return std::max((tallest + 4) * row, cells / rate) + 1e-3 * cells / rate;
 }
 void choose_geometry(swb_server *sv) {
     bool pair = sv->precision == SWB_F32 || sv->precision == SWB_F16;
     for (Req *r : sv->active) pair = pair && r->p.Lx % 2 == 0 && swb::pair_form_ok(r->a);
-    sv->nt = swb::kBatchNT;
-    const int cap = sv->geo_rows > 0 ? sv->geo_rows : kServePairRows;
-    if (pair)
-        sv->nt = sv->geo_nt != 0 ? sv->geo_nt
-                                 : (padded_cells(sv->active, -32, cap) < padded_cells(sv->active, -64, cap)
-                                        ? -32
-                                        : -64);
-    for (Req *r : sv->active) {
-        const int h = pair ? balanced_rows(r->p.Ly, cap) : std::min(swb::kBatchRows, r->p.Ly);
-        swb::set_geometry(r->a, sv->nt, std::max(h, swb::kMinRows));
+    int best_nt = swb::kBatchNT, best_cap = kServePairRows;
+    double best = -1.0;
+    for (int nt : {-64, -32, swb::kBatchNT}) {
+        if ((nt < 0) != pair || (pair && sv->geo_nt != 0 && nt != sv->geo_nt)) continue;
+        for (int cap : {64, 48, 32, 24, 16, 12, 8, 6, 4, 3, 2}) {
+            if (pair && sv->geo_rows > 0) cap = sv->geo_rows;
+            if (!pair && cap > swb::kBatchRows) continue;
+            const double us = iteration_us(sv, nt, cap);
+            if (best < 0.0 || us < best) {
+                best = us;
+                best_nt = nt;
+                best_cap = cap;
+            }
+        }
     }
+    sv->nt = best_nt;
+    for (Req *r : sv->active)
+        swb::set_geometry(r->a, sv->nt, std::max(balanced_rows(r->p.Ly, best_cap), swb::kMinRows));
 }
 
 // Packed table of (lattice, strip) entries, the lattices' reducers first.
