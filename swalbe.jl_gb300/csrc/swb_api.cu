@@ -524,8 +524,7 @@ int plain_iteration(swb_state *s) {
         CUDA_TRY(&s->err, swb::plain_inclination(ps, s->ax, s->ay, fac, s->stream));
     }
     CUDA_TRY(&s->err, swb::plain_equilibrium(ps, p.g, s->stream));
-    CUDA_TRY(&s->err, swb::plain_collide(ps, 1.0 - 1.0 / p.tau, 1.0 / p.tau, s->stream));
-    CUDA_TRY(&s->err, swb::plain_stream(ps, s->stream));
+    CUDA_TRY(&s->err, swb::plain_bgk_stream(ps, 1.0 - 1.0 / p.tau, 1.0 / p.tau, s->stream));
     CUDA_TRY(&s->err, swb::plain_moments(ps, s->stream));
     s->steps++;
     return SWB_OK;
@@ -1051,9 +1050,8 @@ int swb_set_field(swb_state *s, int field, const double *host) {
             default: return fail(&s->err, SWB_ERR_ARG, "unknown field");
         }
         CUDA_TRY(&s->err, cudaMemcpyAsync(dst, host, n * 8, cudaMemcpyHostToDevice, s->stream));
-        // the reference's fout and ftemp are equal between steps
-        if (field == SWB_FIELD_FOUT)
-            CUDA_TRY(&s->err, cudaMemcpyAsync(ps.ftemp, host, n * 8, cudaMemcpyHostToDevice, s->stream));
+        // (the reference's ftemp equals fout between steps: ps.ftemp is only the
+        // buffer the next BGKandStream! writes)
         CUDA_TRY(&s->err, cudaStreamSynchronize(s->stream));
         return SWB_OK;
     }
@@ -1650,8 +1648,7 @@ int swb_op_equilibrium(swb_state *s) {
 }
 int swb_op_bgk_stream(swb_state *s) {
     PLAIN_ONLY(s);
-    CUDA_TRY(&s->err, swb::plain_collide(s->ps, 1.0 - 1.0 / s->p.tau, 1.0 / s->p.tau, s->stream));
-    CUDA_TRY(&s->err, swb::plain_stream(s->ps, s->stream));
+    CUDA_TRY(&s->err, swb::plain_bgk_stream(s->ps, 1.0 - 1.0 / s->p.tau, 1.0 / s->p.tau, s->stream));
     return SWB_OK;
 }
 int swb_op_moments(swb_state *s) {

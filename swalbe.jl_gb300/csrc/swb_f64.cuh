@@ -189,16 +189,14 @@ __device__ __forceinline__ void grad64(O &o, const Near64 &v, double &gx, double
                o.mul(1.0 / 12.0, o.sub(o.sub(o.add(v.ipjp, v.imjp), v.imjm), v.ipjm)));
 }
 
-// -h ∇p - slip (src/simulate.jl:18-19) with slippage!'s
-// (6 μ h u) / (2 h^2 + 6 δ h + 3 δ^2) (src/forcing.jl:43-44).
+// slippage! (src/forcing.jl:43-44): (6 μ h u) / (2 h^2 + 6 δ h + 3 δ^2).
 template <class O>
-__device__ __forceinline__ void force64(O &o, double h, double ux, double uy, double gx, double gy,
-                                        double mu6, double delta6, double delta3sq, double &Fx, double &Fy) {
+__device__ __forceinline__ void slip64(O &o, double h, double ux, double uy, double mu6, double delta6,
+                                       double delta3sq, double &sx, double &sy) {
     const double den = o.add(o.twice_plus(o.muln(h, h), o.mul(delta6, h)), delta3sq);
     const double mh = o.mul(mu6, h), y = o.recip(den);
-    const double sx = o.quot(o.mul(mh, ux), den, y), sy = o.quot(o.mul(mh, uy), den, y);
-    Fx = o.sub(-o.mul(h, gx), sx);
-    Fy = o.sub(-o.mul(h, gy), sy);
+    sx = o.quot(o.mul(mh, ux), den, y);
+    sy = o.quot(o.mul(mh, uy), den, y);
 }
 
 // equilibrium! (src/equilibrium.jl:67-114); g56 = 5/6 g, g15 = 1.5 g.  G0: no

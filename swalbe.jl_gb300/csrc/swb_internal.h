@@ -356,8 +356,7 @@ cudaError_t plain_thermal(const PlainState &s, double k6, double delta, unsigned
 cudaError_t plain_inclination(const PlainState &s, double ax, double ay, double fac,
                               cudaStream_t st);
 cudaError_t plain_equilibrium(const PlainState &s, double g, cudaStream_t st);
-cudaError_t plain_collide(const PlainState &s, double omeg, double invtau, cudaStream_t st);
-cudaError_t plain_stream(const PlainState &s, cudaStream_t st);
+cudaError_t plain_bgk_stream(PlainState &s, double omeg, double invtau, cudaStream_t st);  // exchanges fout and ftemp
 cudaError_t plain_moments(const PlainState &s, cudaStream_t st);
 
 // Measures of a Float64/float height field: block partials + last-block

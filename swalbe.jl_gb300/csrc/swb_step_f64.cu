@@ -236,9 +236,11 @@ struct CollideIn {
 template <bool TAU1, bool G0, bool GEN, class O>
 __device__ __forceinline__ void collide64(O &o, const StepArgs &a, const Cell64 &x, const CollideIn &v,
                                           double out[9]) {
-    double gx, gy, Fx, Fy, fe[9];
+    double gx, gy, sx, sy, fe[9];
     grad64(o, v.p, gx, gy);
-    force64(o, v.h, v.ux, v.uy, gx, gy, x.mu6, x.delta6, x.delta3sq, Fx, Fy);
+    slip64(o, v.h, v.ux, v.uy, x.mu6, x.delta6, x.delta3sq, sx, sy);
+    // the force sum (src/simulate.jl:18-19)
+    double Fx = o.sub(-o.mul(v.h, gx), sx), Fy = o.sub(-o.mul(v.h, gy), sy);
     if (GEN && a.thermal) {  // Fx .= -h∇px .- slipx .- kbtx (scripts/Rivulet_stability.jl:123)
         Fx = o.sub(Fx, v.kx);
         Fy = o.sub(Fy, v.ky);
@@ -620,12 +622,38 @@ __device__ __forceinline__ Nb neighbours(long long c, int Lx, int Ly) {
     return n;
 }
 
+__device__ __forceinline__ Near64 near_of(const double *v, const Nb &b) {
+    return {v[b.ip], v[b.jp], v[b.im], v[b.jm], v[b.ipjp], v[b.imjp], v[b.imjm], v[b.ipjm]};
+}
+
+// An op's cell with the integer unit's help (Fast64), and out of line again in
+// Float64 where that met a number it does not hold.  f(o, r): the op with
+// operations o and results r[0 .. K).
+template <int K, class F>
+__device__ __noinline__ void plain_again(const F &f, double *r) {
+    Plain64 o;
+    f(o, r);
+}
+template <int K, class F>
+__device__ __forceinline__ void plain_cell(const Fma64 &g, const F &f, double (&r)[K]) {
+    Fast64 o(g);
+    f(o, r);
+    if (o.bad) {
+        const F copy = f;
+        double again[K];
+        plain_again<K>(copy, again);
+#pragma unroll
+        for (int q = 0; q < K; ++q) r[q] = again[q];
+    }
+}
+
 // (sx, sy): offset of a moving θ field (0 for a fixed one)
-__global__ void k_filmpressure(PlainState s, const double *kapF, double kap, double gamma, int n,
-                               int m, double hmin, double hcrit, int sx, int sy) {
+__global__ void k_filmpressure(PlainState s, Fma64 g, const double *kapF, double kap, double gamma,
+                               int n, int m, double hmin, double hcrit, int sx, int sy) {
+    grid_dep_wait();
+    grid_dep_launch();
     PLAIN_LOOP(s) {
         const Nb b = neighbours(c, s.Lx, s.Ly);
-        const double *h = s.h;
         double k = kap;
         if (kapF) {
             int i = (int)(c % s.Lx) - sx, j = (int)(c / s.Lx) - sy;
@@ -633,33 +661,47 @@ __global__ void k_filmpressure(PlainState s, const double *kapF, double kap, dou
             if (j < 0) j += s.Ly;
             k = kapF[(long long)j * s.Lx + i];
         }
-        s.p[c] = pressure_cell<true, double>(h[c], h[b.ip], h[b.jp], h[b.im], h[b.jm], h[b.ipjp],
-                                             h[b.imjp], h[b.imjm], h[b.ipjm], k, gamma, hmin,
-                                             hcrit, n, m);
-    }
-}
-
-__global__ void k_hgradp(PlainState s) {
-    PLAIN_LOOP(s) {
-        const Nb b = neighbours(c, s.Lx, s.Ly);
-        const double *p = s.p;
-        double gx, gy;
-        grad9<double>(p[b.ip], p[b.jp], p[b.im], p[b.jm], p[b.ipjp], p[b.imjp], p[b.imjm],
-                      p[b.ipjm], gx, gy);
-        s.hgx[c] = s.h[c] * gx;
-        s.hgy[c] = s.h[c] * gy;
-    }
-}
-
-__global__ void k_slippage(PlainState s, double delta6, double delta3sq, double mu6) {
-    PLAIN_LOOP(s) {
         const double h = s.h[c];
-        s.sx[c] = (mu6 * h * s.ux[c]) / (2.0 * (h * h) + delta6 * h + delta3sq);
-        s.sy[c] = (mu6 * h * s.uy[c]) / (2.0 * (h * h) + delta6 * h + delta3sq);
+        const Near64 v = near_of(s.h, b);
+        double r[1];
+        plain_cell<1>(g, [=](auto &o, double *p) { p[0] = pressure64(o, h, v, k, gamma, hmin, hcrit, n, m); }, r);
+        s.p[c] = r[0];
     }
 }
 
-__global__ void k_force_sum(PlainState s) {
+__global__ void k_hgradp(PlainState s, Fma64 g) {
+    grid_dep_wait();
+    grid_dep_launch();
+    PLAIN_LOOP(s) {
+        const Near64 v = near_of(s.p, neighbours(c, s.Lx, s.Ly));
+        const double h = s.h[c];
+        double r[2];
+        plain_cell<2>(g, [=](auto &o, double *q) {
+            double gx, gy;
+            grad64(o, v, gx, gy);
+            q[0] = o.mul(h, gx);
+            q[1] = o.mul(h, gy);
+        }, r);
+        s.hgx[c] = r[0];
+        s.hgy[c] = r[1];
+    }
+}
+
+__global__ void k_slippage(PlainState s, Fma64 g, double delta6, double delta3sq, double mu6) {
+    grid_dep_wait();
+    grid_dep_launch();
+    PLAIN_LOOP(s) {
+        const double h = s.h[c], ux = s.ux[c], uy = s.uy[c];
+        double r[2];
+        plain_cell<2>(g, [=](auto &o, double *q) { slip64(o, h, ux, uy, mu6, delta6, delta3sq, q[0], q[1]); }, r);
+        s.sx[c] = r[0];
+        s.sy[c] = r[1];
+    }
+}
+
+__global__ void k_force_sum(PlainState s, Fma64) {
+    grid_dep_wait();
+    grid_dep_launch();
     PLAIN_LOOP(s) {
         s.Fx[c] = -s.hgx[c] - s.sx[c];
         s.Fy[c] = -s.hgy[c] - s.sy[c];
@@ -668,8 +710,10 @@ __global__ void k_force_sum(PlainState s) {
 
 // Fx .-= kbtx, Fy .-= kbty with thermal!'s forces of iteration t
 // (src/forcing.jl:297-311; the force sum of scripts/Rivulet_stability.jl:123).
-__global__ void k_thermal(PlainState s, double k6, double delta, unsigned long long seed,
+__global__ void k_thermal(PlainState s, Fma64, double k6, double delta, unsigned long long seed,
                           long long t) {
+    grid_dep_wait();
+    grid_dep_launch();
     PLAIN_LOOP(s) {
         double kx, ky;
         thermal_force<true, double>(seed, c, t, k6, s.h[c], delta, &kx, &ky);
@@ -678,63 +722,101 @@ __global__ void k_thermal(PlainState s, double k6, double delta, unsigned long l
     }
 }
 
-__global__ void k_inclination(PlainState s, double ax, double ay, double fac) {
+__global__ void k_inclination(PlainState s, Fma64, double ax, double ay, double fac) {
+    grid_dep_wait();
+    grid_dep_launch();
     PLAIN_LOOP(s) {
         s.Fx[c] = s.Fx[c] + (s.h[c] * ax) * fac;
         s.Fy[c] = s.Fy[c] + (s.h[c] * ay) * fac;
     }
 }
 
-__global__ void k_equilibrium(PlainState s, double g) {
+template <bool G0>
+__global__ void k_equilibrium(PlainState s, Fma64 g, double g56, double g15) {
+    grid_dep_wait();
+    grid_dep_launch();
     PLAIN_LOOP(s) {
-        double fe[9];
-        const double ux = s.ux[c], uy = s.uy[c];
-        feq_literal<double>(s.h[c], ux, uy, g, fe);
-        s.vsq[c] = ux * ux + uy * uy;
-        for (int q = 0; q < 9; ++q) s.feq[q * s.N + c] = fe[q];
+        const double h = s.h[c], ux = s.ux[c], uy = s.uy[c];
+        double r[10];
+        plain_cell<10>(g, [=](auto &o, double *q) {
+            double fe[9];
+            feq64<G0>(o, h, ux, uy, g56, g15, fe);
+            for (int k = 0; k < 9; ++k) q[k] = fe[k];
+            q[9] = o.add(o.mul(ux, ux), o.mul(uy, uy));
+        }, r);
+        s.vsq[c] = r[9];
+#pragma unroll
+        for (int q = 0; q < 9; ++q) s.feq[q * s.N + c] = r[q];
     }
 }
 
-__global__ void k_collide(PlainState s, double omeg, double invtau) {
-    PLAIN_LOOP(s) {
-        const double Fx = s.Fx[c], Fy = s.Fy[c];
-        for (int q = 0; q < 9; ++q) {
-            double v = omeg * s.ftemp[q * s.N + c] + invtau * s.feq[q * s.N + c];
-            if (q > 0) v = v + source<double>(q, Fx, Fy);
-            s.fout[q * s.N + c] = v;
-        }
-    }
-}
-
-__global__ void k_stream(PlainState s) {  // circshift!(ft_q, fo_q, c_q)
+// BGKandStream! in one pass: the collision of every cell, each population
+// stored where it streams to (circshift!(ft_q, fo_q, c_q)).  The reference's
+// ftemp equals its fout between ops, so the other buffer takes the result
+// and the caller exchanges the two.
+__global__ void k_bgk_stream(PlainState s, Fma64 g, double omeg, double invtau) {
     const int CX[9] = {0, 1, 0, -1, 0, 1, -1, -1, 1};
     const int CY[9] = {0, 0, 1, 0, -1, 1, 1, -1, -1};
+    grid_dep_wait();
+    grid_dep_launch();
     PLAIN_LOOP(s) {
-        const int i = (int)(c % s.Lx), j = (int)(c / s.Lx);
+        const double Fx = s.Fx[c], Fy = s.Fy[c];
+        struct {
+            double f[9], fe[9];
+        } v;
+#pragma unroll
         for (int q = 0; q < 9; ++q) {
-            const int si = wrapc(i - CX[q], s.Lx), sj = wrapc(j - CY[q], s.Ly);
-            s.ftemp[q * s.N + c] = s.fout[q * s.N + (long long)sj * s.Lx + si];
+            v.f[q] = s.fout[q * s.N + c];
+            v.fe[q] = s.feq[q * s.N + c];
+        }
+        double r[9];
+        plain_cell<9>(g, [=](auto &o, double *out) {
+            double w[9];
+            relax64<false>(o, v.fe, v.f, omeg, invtau, Fx, Fy, w);
+            for (int q = 0; q < 9; ++q) out[q] = w[q];
+        }, r);
+        const int i = (int)(c % s.Lx), j = (int)(c / s.Lx);
+#pragma unroll
+        for (int q = 0; q < 9; ++q) {
+            const int di = wrapc(i + CX[q], s.Lx), dj = wrapc(j + CY[q], s.Ly);
+            s.ftemp[q * s.N + (long long)dj * s.Lx + di] = r[q];
         }
     }
 }
 
-__global__ void k_moments(PlainState s) {
+__global__ void k_moments(PlainState s, Fma64 g) {
+    grid_dep_wait();
+    grid_dep_launch();
     PLAIN_LOOP(s) {
-        double f[9], h, jx, jy, ux, uy;
-        for (int q = 0; q < 9; ++q) f[q] = s.fout[q * s.N + c];
-        moments9<true>(f, h, jx, jy);
-        velocity<true>(h, jx, jy, ux, uy);
-        s.h[c] = h;
-        s.ux[c] = ux;
-        s.uy[c] = uy;
+        struct {
+            double f[9];
+        } v;
+#pragma unroll
+        for (int q = 0; q < 9; ++q) v.f[q] = s.fout[q * s.N + c];
+        double r[3];
+        plain_cell<3>(g, [=](auto &o, double *q) {
+            double h, jx, jy;
+            moments64(o, v.f, h, jx, jy);
+            const double y = o.recip(h);
+            q[0] = h;
+            q[1] = o.quot(jx, h, y);
+            q[2] = o.quot(jy, h, y);
+        }, r);
+        s.h[c] = r[0];
+        s.ux[c] = r[1];
+        s.uy[c] = r[2];
     }
 }
 
-#define PLAIN_LAUNCH(kernel, s, st, ...)                                  \
-    do {                                                                  \
-        count_launches(1);                                                \
-        kernel<<<grid_for((s).N, 256), 256, 0, st>>>(s, ##__VA_ARGS__);   \
-        return cudaGetLastError();                                        \
+// Blocks of 64 threads: a lattice of 128 x 96 cells then has a warp for every SM
+// quarter, where blocks of 256 kept two thirds of the SMs idle.  The launches
+// overlap (launch_step): an op's kernel after another takes 4.1 us without
+// that, however short it is.
+constexpr int kPlainNT = 64;
+#define PLAIN_LAUNCH(kernel, s, st, ...)                                                               \
+    do {                                                                                               \
+        count_launches(1);                                                                             \
+        return launch_step(kernel, grid_for((s).N, kPlainNT), kPlainNT, st, s, Fma64{1.0, -0.0}, ##__VA_ARGS__); \
     } while (0)
 
 cudaError_t plain_filmpressure(const PlainState &s, const double *kapF, double kap, double gamma,
@@ -758,19 +840,19 @@ cudaError_t plain_inclination(const PlainState &s, double ax, double ay, double 
     PLAIN_LAUNCH(k_inclination, s, st, ax, ay, fac);
 }
 cudaError_t plain_equilibrium(const PlainState &s, double g, cudaStream_t st) {
-    PLAIN_LAUNCH(k_equilibrium, s, st, g);
+    auto *const kern = g == 0.0 ? k_equilibrium<true> : k_equilibrium<false>;
+    PLAIN_LAUNCH(kern, s, st, (5.0 / 6.0) * g, 1.5 * g);
 }
-cudaError_t plain_collide(const PlainState &s, double omeg, double invtau, cudaStream_t st) {
-    PLAIN_LAUNCH(k_collide, s, st, omeg, invtau);
-}
-cudaError_t plain_stream(const PlainState &s, cudaStream_t st) {
+cudaError_t plain_bgk_stream(PlainState &s, double omeg, double invtau, cudaStream_t st) {
     count_launches(1);
-    k_stream<<<grid_for(s.N, 256), 256, 0, st>>>(s);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    // fout .= ftemp (src/collide.jl:103)
-    return cudaMemcpyAsync(s.fout, s.ftemp, 9 * s.N * sizeof(double), cudaMemcpyDeviceToDevice,
-                           st);
+    const cudaError_t e = launch_step(k_bgk_stream, grid_for(s.N, kPlainNT), kPlainNT, st, s,
+                                      Fma64{1.0, -0.0}, omeg, invtau);
+    if (e == cudaSuccess) {
+        double *f = s.fout;
+        s.fout = s.ftemp;
+        s.ftemp = f;
+    }
+    return e;
 }
 cudaError_t plain_moments(const PlainState &s, cudaStream_t st) { PLAIN_LAUNCH(k_moments, s, st); }
 
