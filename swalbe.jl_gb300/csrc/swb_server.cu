@@ -190,27 +190,35 @@ int balanced_rows(int Ly, int cap) {
     return (Ly + strips - 1) / strips;
 }
 // Estimated time of an iteration with strips of geometry nt and at most cap
-// rows: the march of the tallest strip at one row's latency, or the padded
-// cells at the full GPU's rate, whichever is longer.  The constants were
-// measured on GB300: a lone pair strip of 64 rows takes 49 us (0.7 us per
-// row), a full resident set runs 80 cells per ns; one-column strips 0.6 us and
-// 55; Float64 strips 10 us and 2.  (Eight lattices of 32k to 147k cells: 50 us
-// per iteration with 64 rows.)
-double iteration_us(const swb_server *sv, int nt, int cap) {
-    const bool f64 = sv->precision == SWB_F64;
-    const double row = nt < 0 ? 0.7 : (f64 ? 10.0 : 0.6), rate = nt < 0 ? 80e3 : (f64 ? 2e3 : 55e3);
+// rows.  Pair strips: launch and drain, then waves of up to 8 CTAs of 64
+// threads (16 of 32) per SM, each as long as a march over the tallest strip,
+// whose rows take 0.655 us alone on an SM and 2.1 times that in a full wave
+// (measured on GB300: 64 to 4M cells in 1 to 32 lattices, 18 geometries each;
+// the estimate is within 20 % of all, and the one it picks within 15 % of the
+// best).  E.g. a 1024² lattice 50.7 us with 64 rows, 21.0 with 8; eight of 32k
+// to 147k cells 51.1 and 17.7 (60 columns, 6 rows).  One-column strips: the
+// march at 0.6 us per row (Float64: 10) or 55 cells per ns (2).
+double iteration_us(const swb_server *sv, int nt, int cap, int sms) {
     const int w = nt < 0 ? -2 * nt - 4 : nt - 4;
-    double cells = 0.0;
+    double strips = 0.0, cells = 0.0;
     int tallest = 0;
     for (const Req *r : sv->active) {
         const int h = balanced_rows(r->p.Ly, cap);
+        const double n = (double)((r->p.Lx + w - 1) / w) * (double)((r->p.Ly + h - 1) / h);
         tallest = std::max(tallest, h);
-        cells += (double)((r->p.Lx + w - 1) / w) * (w + 4) * (double)((r->p.Ly + h - 1) / h) * (h + 4);
+        strips += n;
+        cells += n * (w + 4) * (h + 4);
     }
-    // (the small term lets fewer cells decide between equal marches)
-    return std::max((tallest + 4) * row, cells / rate) + 1e-3 * cells / rate;
+    if (nt >= 0) {
+        const bool f64 = sv->precision == SWB_F64;
+        return std::max((tallest + 4) * (f64 ? 10.0 : 0.6), cells / (f64 ? 2e3 : 55e3));
+    }
+    const double c = strips * (-nt / 64.0) / sms;  // CTAs per SM, in units of 64 threads
+    auto row = [](double c) { return 0.655 * (1.0 + 0.17 * std::max(0.0, c - 1.4)); };
+    const double waves = std::floor(c / 8.0), rest = c - 8.0 * waves;
+    return 4.7 + (tallest + 4) * (waves * row(8.0) + (rest > 0.0 ? row(rest) : 0.0));
 }
-void choose_geometry(swb_server *sv) {
+void choose_geometry(swb_server *sv, int sms) {
     bool pair = sv->precision == SWB_F32 || sv->precision == SWB_F16;
     for (Req *r : sv->active) pair = pair && r->p.Lx % 2 == 0 && swb::pair_form_ok(r->a);
     int best_nt = swb::kBatchNT, best_cap = kServePairRows;
@@ -220,7 +228,7 @@ void choose_geometry(swb_server *sv) {
         for (int cap : {64, 48, 32, 24, 16, 12, 8, 6, 4, 3, 2}) {
             if (pair && sv->geo_rows > 0) cap = sv->geo_rows;
             if (!pair && cap > swb::kBatchRows) continue;
-            const double us = iteration_us(sv, nt, cap);
+            const double us = iteration_us(sv, nt, cap, sms);
             if (best < 0.0 || us < best) {
                 best = us;
                 best_nt = nt;
@@ -264,8 +272,8 @@ bool put_table(swb_server *sv, const std::vector<T> &v, T **d, size_t *cap) {
 
 // The tables of the resident set (and, for pair strips, of its one-column
 // fallback strips), uploaded on the tick stream.
-bool upload_table(swb_server *sv) {
-    choose_geometry(sv);
+bool upload_table(swb_server *sv, int sms) {
+    choose_geometry(sv, sms);
     std::vector<StepArgs> args;
     for (Req *r : sv->active) args.push_back(r->a);
     const std::vector<TileRef> tiles = tile_table(args);
@@ -371,7 +379,7 @@ void worker_main(swb_server *sv) {
             sv->geo_nt = sv->want_nt;
             sv->geo_rows = sv->want_rows;
         }
-        if (changed && !sv->active.empty() && !upload_table(sv)) {
+        if (changed && !sv->active.empty() && !upload_table(sv, sms)) {
             set_error(sv, "tile table upload failed");
             std::this_thread::sleep_for(std::chrono::milliseconds(10));
             continue;
