@@ -534,15 +534,20 @@ constexpr int kGraphSteps = 64;
 
 // Geometries chosen by the autotuner, per (Lx, Ly, precision), process-wide.
 std::mutex g_tune_mu;
-std::vector<std::array<int, 7>> g_tuned;  // Lx, Ly, precision, mode, nt, h, persist
+std::vector<std::array<int, 8>> g_tuned;  // Lx, Ly, precision, mode, kind, nt, h, persist
 
-bool tuned_lookup(int Lx, int Ly, int prec, int mode, int *nt, int *h, bool *persist) {
+// What of a step decides which kernels run it: τ = 1, the kind of θ, forces.
+int step_kind(const StepArgs &a) {
+    return a.theta_mode | (a.tau_is_one ? 4 : 0) | (a.incl ? 8 : 0) | (a.thermal ? 16 : 0);
+}
+
+bool tuned_lookup(int Lx, int Ly, int prec, int mode, int kind, int *nt, int *h, bool *persist) {
     std::lock_guard<std::mutex> g(g_tune_mu);
     for (auto &e : g_tuned)
-        if (e[0] == Lx && e[1] == Ly && e[2] == prec && e[3] == mode) {
-            *nt = e[4];
-            *h = e[5];
-            *persist = e[6] != 0;
+        if (e[0] == Lx && e[1] == Ly && e[2] == prec && e[3] == mode && e[4] == kind) {
+            *nt = e[5];
+            *h = e[6];
+            *persist = e[7] != 0;
             return true;
         }
     return false;
@@ -563,11 +568,11 @@ int sm_count() {
 
 // Rows of resident tiles for a lattice: the shortest tiles (the most CTAs)
 // whose CTAs are all co-resident; 0 when even kResMaxTH rows do not fit.
-int resident_rows(int Lx, int Ly, int precision, int nt = swb::kResGeom) {
+int resident_rows(int Lx, int Ly, int precision, bool gen, int nt = swb::kResGeom) {
     const long long tx = (Lx + swb::kResTW - 1) / swb::kResTW, sms = sm_count();
     for (int h = 1; h <= swb::kResMaxTH; ++h) {
         const long long tiles = tx * ((Ly + h - 1) / h);
-        const int per_sm = swb::resident_blocks_per_sm(precision, h, nt);
+        const int per_sm = swb::resident_blocks_per_sm(precision, h, gen, nt);
         if (per_sm > 0 && tiles <= per_sm * sms) return h < Ly ? h : Ly;
     }
     return 0;
@@ -579,7 +584,8 @@ int resident_rows(int Lx, int Ly, int precision, int nt = swb::kResGeom) {
 int run_grid(swb_state *s) {
     const long long tiles = (long long)s->a.tiles_x * s->a.tiles_y;
     if (swb::resident_geometry(s->a.march_nt)) {
-        const int per_sm = swb::resident_blocks_per_sm(s->precision, s->a.march_h, s->a.march_nt);
+        const int per_sm = swb::resident_blocks_per_sm(s->precision, s->a.march_h, swb::step_general(s->a),
+                                                       s->a.march_nt);
         return (per_sm > 0 && tiles <= (long long)per_sm * sm_count()) ? (int)tiles : 0;
     }
     const int per_sm = swb::fused_run_blocks_per_sm(s->precision, s->a.march_nt);
@@ -706,7 +712,7 @@ float tune_probe(swb_state *s, cudaEvent_t e0, cudaEvent_t e1) {
 int autotune_geometry(swb_state *s, long long &left) {
     int nt = 0, h = 0;
     bool pers = false;
-    if (tuned_lookup(s->p.Lx, s->p.Ly, s->precision, s->mode, &nt, &h, &pers)) {
+    if (tuned_lookup(s->p.Lx, s->p.Ly, s->precision, s->mode, step_kind(s->a), &nt, &h, &pers)) {
         swb::set_geometry(s->a, nt, h);
         s->persist = pers;
         s->invalidate_graph();
@@ -733,7 +739,7 @@ int autotune_geometry(swb_state *s, long long &left) {
     // shared memory: the shortest co-resident tiles
     if (multi_ok && swb::resident_ok(s->a)) {
         for (int rg : {swb::kResGeom, swb::kResGeom2}) {
-            const int res_h = resident_rows(s->p.Lx, s->p.Ly, s->precision, rg);
+            const int res_h = resident_rows(s->p.Lx, s->p.Ly, s->precision, swb::step_general(s->a), rg);
             if (res_h > 0) todo.push_back({rg, res_h, 1});
         }
     }
@@ -781,7 +787,7 @@ int autotune_geometry(swb_state *s, long long &left) {
     s->tuned = true;
     if (rc == SWB_OK) {
         std::lock_guard<std::mutex> g(g_tune_mu);
-        g_tuned.push_back({s->p.Lx, s->p.Ly, s->precision, s->mode, bnt, bh, bpers ? 1 : 0});
+        g_tuned.push_back({s->p.Lx, s->p.Ly, s->precision, s->mode, step_kind(s->a), bnt, bh, bpers ? 1 : 0});
     }
     return rc;
 }
@@ -1251,14 +1257,14 @@ int swb_set_geometry(swb_state *s, int nt, int h) {
     } else if (swb::resident_geometry(nt)) {
         if (s->precision != SWB_F32 && s->precision != SWB_F16)
             return fail(&s->err, SWB_ERR_UNSUPPORTED, "resident tiles: FP32 and FP16 storage only");
-        if (h == 0) h = resident_rows(s->p.Lx, s->p.Ly, s->precision, nt);
+        if (h == 0) h = resident_rows(s->p.Lx, s->p.Ly, s->precision, swb::step_general(s->a), nt);
         if (h < 1 || h > swb::kResMaxTH)
             return fail(&s->err, SWB_ERR_UNSUPPORTED,
                         "resident tiles: the lattice does not fit in the GPU's shared memory "
                         "(rows must be 1..40 with every tile co-resident)");
         const long long tiles = (long long)((s->p.Lx + swb::kResTW - 1) / swb::kResTW) *
                                 ((s->p.Ly + h - 1) / h);
-        if (tiles > (long long)swb::resident_blocks_per_sm(s->precision, h, nt) * sm_count())
+        if (tiles > (long long)swb::resident_blocks_per_sm(s->precision, h, swb::step_general(s->a), nt) * sm_count())
             return fail(&s->err, SWB_ERR_UNSUPPORTED,
                         "resident tiles: more tiles than the GPU holds at once; use more rows");
     } else if (swb::pair_geometry(nt)) {

@@ -320,11 +320,11 @@ int batch_blocks_per_sm_f64(int nt);
 // that hold it (0: not possible), and n iterations in one cooperative launch
 // of tiles_x * tiles_y CTAs (closes the sequence itself).
 size_t resident_smem_bytes(int h, int nt = kResGeom);
-int resident_blocks_per_sm(int precision, int h, int nt = kResGeom);
+int resident_blocks_per_sm(int precision, int h, bool gen, int nt = kResGeom);
 cudaError_t launch_resident_run(int precision, const StepArgs &a, int n, cudaStream_t st);
-// Whether iterations of `a` may run as resident tiles (the common steady
-// τ = 1 step with scalar θ of an FP32-arithmetic lattice).
-inline bool resident_ok(const StepArgs &a) { return a.tau_is_one && !step_general(a); }
+// Whether steady iterations of `a` may run as resident tiles (τ = 1 steps of
+// an FP32-arithmetic lattice).
+inline bool resident_ok(const StepArgs &a) { return a.tau_is_one; }
 // Resident CTAs per SM of the pair-strip kernel (FP32 / FP16 storage).
 int pair_blocks_per_sm(int precision, int nt);
 // Rows per pair strip for a lattice: the strip march takes about the same

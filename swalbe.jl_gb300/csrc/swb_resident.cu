@@ -18,9 +18,11 @@
 // then all CTAs meet at the bounded grid barrier of the multi-step kernel.
 // The per-cell arithmetic is the strip march's (moments9, pressure_cell,
 // grad9, force_fast, collide_fast), so results are bit-identical to it; the
-// measures go through the same integer accumulators and reducer.  The common
-// steady τ = 1 step only (scalar θ, no rare forces): the host runs every
-// other iteration on strips.
+// measures go through the same integer accumulators and reducer.  The steady
+// τ = 1 step only; GEN compiles in θ fields, the θ wave, thermal noise and the
+// inclination (384 x 250, per iteration: with an inclination 6.5 us against 7.3
+// for the best strips, with a θ field 7.0 against 7.6; without either, and
+// without GEN, 5.7 against 5.9).  The host runs every other iteration on strips.
 #include <type_traits>
 
 #include "swb_step_impl.cuh"
@@ -74,10 +76,12 @@ __device__ __forceinline__ bool res_wait(unsigned int *ctr, int *err, unsigned i
     return __syncthreads_and(ok) != 0;
 }
 
-template <class S, int NT>
+template <class S, int NT, bool GEN>
 __global__ void __launch_bounds__(NT, kResThreads / NT) resident_run_kernel(const StepArgs a, int n) {
     using R = float;
     extern __shared__ __align__(16) float dsm[];
+    // κ and cos θ of the tile's columns (one ring for κ) in the θ wave
+    __shared__ float wave_kap[GEN ? kPW : 1], wave_cos[GEN ? kPW : 1];
     const int TH = a.march_h;
     const int PL = (TH + 6) * kEW;  // one population plane of the region
     float *F = dsm;                 // [9][TH + 6][kEW]
@@ -101,6 +105,7 @@ __global__ void __launch_bounds__(NT, kResThreads / NT) resident_run_kernel(cons
     const bool measure = a.meas_mask || a.mass_corr;
     const R gamma = R(a.gamma), hmin = R(a.hmin), hcrit = R(a.hcrit), kap = R(a.kap);
     const R thr = R(a.hthresh);
+    const int mode = GEN ? a.theta_mode : (int)THETA_SCALAR;
 
     // Populations of the region from the buffer iteration done + 1 pulls
     // from (L2 loads: other CTAs wrote them in this launch); ring_only:
@@ -146,6 +151,15 @@ __global__ void __launch_bounds__(NT, kResThreads / NT) resident_run_kernel(cons
                 load(done, true);
             }
         }
+        int fsx = 0, fsy = 0;  // offset of a moving θ field
+        if (mode == THETA_FIELD) substrate_shift(a, tt, &fsx, &fsy);
+        if (mode == THETA_WAVE && t >= 32 && t < 32 + kPW) {
+            const KapCos<R> w = wave_at<R>(a, wrapc(X0 - 33 + t, Lx), tt);
+            wave_kap[t - 32] = w.kap;
+            wave_cos[t - 32] = w.cs;
+        }
+        // index into the θ field of column x and row y
+        auto field = [&](int x, int y) { return wrapc(y - fsy, Ly) * Lx + wrapc(x - fsx, Lx); };
         __syncthreads();
         // A. pull and moments on the tile and 2 rings
         {
@@ -184,9 +198,14 @@ __global__ void __launch_bounds__(NT, kResThreads / NT) resident_run_kernel(cons
                 const int px = i % kPW, py = i / kPW;
                 if (px >= w1) continue;
                 const float *hc = Hs + (py + 1) * kHW + (px + 1), *hm = hc - kHW, *hp = hc + kHW;
+                R kp = kap;
+                if (mode == THETA_FIELD)
+                    kp = reinterpret_cast<const R *>(a.kapF)[field(X0 - 1 + px, Y0 - 1 + py)];
+                else if (mode == THETA_WAVE)
+                    kp = wave_kap[px];
                 // ip = h[i-1,j], jp = h[i,j-1], im = h[i+1,j], jm = h[i,j+1], ...
                 Ps[py * kPW + px] = pressure_cell<false, R>(hc[0], hc[-1], hm[0], hc[1], hp[0],
-                                                            hm[-1], hm[1], hp[1], hp[-1], kap,
+                                                            hm[-1], hm[1], hp[1], hp[-1], kp,
                                                             gamma, hmin, hcrit, a.n, a.m);
             }
         }
@@ -209,7 +228,14 @@ __global__ void __launch_bounds__(NT, kResThreads / NT) resident_run_kernel(cons
             velocity<false>(h, JX[o], JY[o], ux, uy);
             const float *pc = Ps + (oy + 1) * kPW + ox + 1, *pm = pc - kPW, *pp = pc + kPW;
             grad9<R>(pc[-1], pm[0], pc[1], pp[0], pm[-1], pm[1], pp[1], pp[-1], gpx, gpy);  // h∇p!
-            const float2 Fv = force_fast(cc, h, ux, uy, gpx, gpy);
+            float2 Fv = force_fast(cc, h, ux, uy, gpx, gpy);
+            if (GEN && a.thermal) {
+                R kx, ky;
+                thermal_force<false, R>(a.seed, (long long)cell, tt, R(a.k6), h, R(a.delta), &kx, &ky);
+                Fv = f2(Fv.x - kx, Fv.y - ky);
+            }
+            if (GEN && a.incl)
+                Fv = f2(__fmaf_rn(h * R(a.ax), cc.incl_fac, Fv.x), __fmaf_rn(h * R(a.ay), cc.incl_fac, Fv.y));
             float fo[9];
             [[maybe_unused]] __half2 hb[4];
             collide_fast<S, false, true>(cc, h, ux, uy, Fv.x, Fv.y, h, nullptr, cell, tt, &LO[o], fo,
@@ -242,6 +268,10 @@ __global__ void __launch_bounds__(NT, kResThreads / NT) resident_run_kernel(cons
                     R gx2, gy2;
                     grad9<R>(hc[-1], hm[0], hc[1], hp[0], hm[-1], hm[1], hp[1], hp[-1], gx2, gy2);
                     area_add(part, R(sqrt(gx2 * gx2 + gy2 * gy2 + R(1))));
+                    if (mode == THETA_FIELD)
+                        cos_add(part, reinterpret_cast<const R *>(a.cosF)[field(X0 + ox, Y0 + oy)]);
+                    else if (mode == THETA_WAVE)
+                        cos_add(part, wave_cos[ox + 1]);
                 }
             }
         }
@@ -290,21 +320,24 @@ __global__ void __launch_bounds__(NT, kResThreads / NT) resident_run_kernel(cons
 // Allow the kernel the dynamic shared memory of a tile (a host-side
 // attribute of the current device's context; set before every query or
 // launch, which is cheap and keeps it right on every device).
-template <class S, int NT>
+template <class S, int NT, bool GEN>
 cudaError_t prepare(size_t bytes) {
-    return cudaFuncSetAttribute(resident_run_kernel<S, NT>,
+    return cudaFuncSetAttribute(resident_run_kernel<S, NT, GEN>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-// Runs f(store tag, threads) for a precision and resident geometry.
+// Runs f(store tag, threads, general) for a precision and resident geometry.
 template <class F>
-cudaError_t res_dispatch(int precision, int nt, F &&f) {
+cudaError_t res_dispatch(int precision, int nt, bool gen, F &&f) {
+    auto by_gen = [&](auto store, auto threads) {
+        return gen ? f(store, threads, std::true_type{}) : f(store, threads, std::false_type{});
+    };
     const bool half = precision == SWB_F16;
     if (nt == kResGeom2)
-        return half ? f(StoreF16T<LdCG>{}, std::integral_constant<int, kResThreads / 2>{})
-                    : f(StoreF32T<LdCG>{}, std::integral_constant<int, kResThreads / 2>{});
-    return half ? f(StoreF16T<LdCG>{}, std::integral_constant<int, kResThreads>{})
-                : f(StoreF32T<LdCG>{}, std::integral_constant<int, kResThreads>{});
+        return half ? by_gen(StoreF16T<LdCG>{}, std::integral_constant<int, kResThreads / 2>{})
+                    : by_gen(StoreF32T<LdCG>{}, std::integral_constant<int, kResThreads / 2>{});
+    return half ? by_gen(StoreF16T<LdCG>{}, std::integral_constant<int, kResThreads>{})
+                : by_gen(StoreF32T<LdCG>{}, std::integral_constant<int, kResThreads>{});
 }
 
 }  // namespace
@@ -314,16 +347,17 @@ size_t resident_smem_bytes(int h, int nt) {
     return res_floats(h) * sizeof(float) + (threads / 32) * (sizeof(PartQ) + sizeof(RedPart));
 }
 
-int resident_blocks_per_sm(int precision, int h, int nt) {
+int resident_blocks_per_sm(int precision, int h, bool gen, int nt) {
     if ((precision != SWB_F32 && precision != SWB_F16) || h < 1 || h > kResMaxTH) return 0;
     const size_t bytes = resident_smem_bytes(h, nt);
     int n = 0;
-    cudaError_t e = res_dispatch(precision, nt, [&](auto store, auto threads) {
+    cudaError_t e = res_dispatch(precision, nt, gen, [&](auto store, auto threads, auto general) {
         using S = decltype(store);
         constexpr int NT = decltype(threads)::value;
-        cudaError_t r = prepare<S, NT>(bytes);
+        constexpr bool GEN = decltype(general)::value;
+        cudaError_t r = prepare<S, NT, GEN>(bytes);
         if (r == cudaSuccess)
-            r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, resident_run_kernel<S, NT>, NT, bytes);
+            r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, resident_run_kernel<S, NT, GEN>, NT, bytes);
         return r;
     });
     return e == cudaSuccess ? n : 0;
@@ -338,12 +372,13 @@ cudaError_t launch_resident_run(int precision, const StepArgs &a, int n, cudaStr
     int steps = n;
     void *params[] = {&args, &steps};
     const dim3 grid((unsigned)(a.tiles_x * a.tiles_y));
-    return res_dispatch(precision, a.march_nt, [&](auto store, auto threads) {
+    return res_dispatch(precision, a.march_nt, step_general(a), [&](auto store, auto threads, auto general) {
         using S = decltype(store);
         constexpr int NT = decltype(threads)::value;
-        cudaError_t r = prepare<S, NT>(bytes);
+        constexpr bool GEN = decltype(general)::value;
+        cudaError_t r = prepare<S, NT, GEN>(bytes);
         if (r == cudaSuccess)
-            r = cudaLaunchCooperativeKernel((const void *)resident_run_kernel<S, NT>, grid, dim3(NT),
+            r = cudaLaunchCooperativeKernel((const void *)resident_run_kernel<S, NT, GEN>, grid, dim3(NT),
                                             params, bytes, st);
         return r;
     });
