@@ -988,7 +988,7 @@ int swb_create(const swb_params *p, int precision, swb_state **out) {
             x.wave = x.p + N;
             x.acc = (unsigned long long *)(x.wave + 2 * (size_t)p->Lx);
             CREATE_TRY(cudaMemsetAsync(x.acc, 0, 2 * swb::kAcc64 * 8, s->stream));
-            x.f = {1.0, -0.0};
+            x.f = {1.0};
             x.mu6 = 6.0 * p->mu;
             x.delta6 = 6.0 * p->delta;
             x.delta3sq = 3.0 * (p->delta * p->delta);

@@ -697,7 +697,7 @@ int swb1d_step(swb1d *b, int64_t nsteps) {
             const int n = std::min(b->per_launch, burst - done);
             swb::D1Part *part =
                 b->rec_cap ? b->d_part + (size_t)done * b->nchunks * (swb::kD1NT / 32) : nullptr;
-            const swb::Fma64 f{1.0, -0.0};
+            const swb::Fma64 f{1.0};
             const cudaError_t e =
                 b->rb == 8 ? swb::launch_step(swb::d1q3_run_kernel<double, swb::D1Ops64>, b->nchunks, swb::kD1NT,
                                               b->stream, b->d_args, b->d_chunks, swb::D1Ops64{f}, b->cur, n, part)

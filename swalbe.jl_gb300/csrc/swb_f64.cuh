@@ -4,9 +4,9 @@
 // oracle bit for bit; what changes is the unit that computes it.  GB300 has
 // one Float64 result per 64 FP32 ones: a Float64 warp instruction occupies its
 // SM quarter's unit for 64 cycles or more, in which the quarter can issue some
-// forty integer instructions.  So about half of a cell's operations, the
-// products and the quotients, are computed with integers while the Float64
-// unit does the sums (Fast64).  Measured: products alone 15 cycles per SM and
+// forty integer instructions.  So the products and the quotients, half of a
+// cell's operations, are computed with integers while the Float64 unit does the
+// sums (Fast64).  Measured: products alone 15 cycles per SM and
 // warp, sums alone 16.5 to 19, one of each 19 together.
 #pragma once
 #include "swb_internal.h"
@@ -16,16 +16,6 @@ namespace swb {
 __device__ __forceinline__ uint32_t hi64(double v) { return (uint32_t)__double2hiint(v); }
 __device__ __forceinline__ uint32_t lo64(double v) { return (uint32_t)__double2loint(v); }
 __device__ __forceinline__ bool finite64(double v) { return (hi64(v) & 0x7ff00000u) != 0x7ff00000u; }
-
-// An approximation y of 1 / b: the hardware's seed (about 2^-20) and one
-// cubic step y (1 + e + e^2), e = 1 - b y, whose own error is e^3; y is then
-// within about half an ulp of 1 / b.
-__device__ __forceinline__ double recip64(double b) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    const double e = __fma_rn(-b, y, 1.0);
-    return __fma_rn(y, __fma_rn(e, e, e), y);
-}
 
 // a b rounded to nearest, of normal numbers or (ZERO) zeros, in integers: the
 // 106-bit product of the significands, its upper 62 or 63 bits with a sticky
@@ -63,37 +53,58 @@ __device__ __forceinline__ double mul64(double a, double b, bool &bad) {
     return __hiloint2double((int)(rh | ((ah ^ bh) & 0x80000000u)), (int)rl);
 }
 
-// a / b rounded to nearest from y = recip64(b): q = a y is within two ulp, and
-// the integer remainder R = A 2^s - B Q of the 53-bit significands (exact
-// modulo 2^64, and |R| < 2^56) says by how many ulp q is off, because q is
-// the nearest iff 2 |R| < B (a quotient of doubles is never half-way between
-// two doubles).  One Float64 instruction instead of about nine.  Sets `bad`
-// where that does not hold: exponents near the ends of the range, a q whose
-// neighbours across a power of two are spaced differently, zero or non-finite
-// b.  A zero a is exact as it is.
-__device__ __forceinline__ double quot64(double a, double b, double y, double nzero, bool &bad) {
-    const double q = __fma_rn(a, y, nzero);
-    const uint32_t ah = hi64(a), al = lo64(a), bh = hi64(b), bl = lo64(b), qh = hi64(q), ql = lo64(q);
-    const uint32_t ea = (ah >> 20) & 0x7ff, eb = (bh >> 20) & 0x7ff, eq = (qh >> 20) & 0x7ff;
-    const bool zero = zero64(a);
-    const uint32_t Bh = (bh & 0xfffff) | 0x100000, Qh = (qh & 0xfffff) | 0x100000;
-    // s is 52 or 53, so the low word of A 2^s is zero and its high word is
-    // A's low word shifted by s - 32
-    const uint32_t s = (ea - eb - eq + 1023 + 20) & 31;
-    const uint64_t bq = (uint64_t)bl * ql;
-    const uint32_t Rh = (al << s) - (uint32_t)(bq >> 32) - Bh * ql - bl * Qh;
+// r ~ 2^115 / B for the 53-bit significand B of b, within 6 units: the FP32
+// reciprocal (2^-22) and two Newton steps r (1 + e), e = 1 - r B, in fixed
+// point, the first with e to 2^-51, the second to 2^-60.
+__device__ __forceinline__ uint64_t recip64(double b) {
+    const uint32_t bh = hi64(b), bl = lo64(b);
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;"
+        : "=f"(y)
+        : "f"(__uint_as_float(0x3f800000u | __funnelshift_l(bl, bh & 0xfffffu, 3))));
+    y = fminf(y, 0x1.fffffep-1f);
+    const uint32_t r0 = ((__float_as_uint(y) & 0x7fffffu) | 0x800000u) << 7;
+    // B 2^11 in two words
+    const uint32_t Bh = __funnelshift_l(bl, (bh & 0xfffffu) | 0x100000u, 11), Bl = bl << 11;
+    const int64_t e = (int64_t)(0x4000000000000000ull - (uint64_t)r0 * Bh - __umulhi(r0, Bl));
+    const int64_t r1 = (int64_t)((uint64_t)r0 << 32) + (((int64_t)(int32_t)r0 * (int32_t)(e >> 11)) >> 19);
+    const uint32_t rh = (uint32_t)(r1 >> 32), rl = (uint32_t)r1;
+    const int32_t e1 = -(int32_t)(rh * Bh + __umulhi(rh, Bl) + __umulhi(rl, Bh));
+    return (uint64_t)(r1 + (((int64_t)(int32_t)rh * e1) >> 30));
+}
+
+// a / b rounded to nearest from r = recip64(b): Q = A r / 2^115, rounded to 53
+// bits, is within 0.52 of the quotient of the significands, and the integer
+// remainder R = A 2^s - B Q (exact modulo 2^64) says whether it is the nearest:
+// that is so iff 2 |R| < B, because a quotient of doubles is never half-way
+// between two doubles.  No Float64 instruction instead of about nine.  Sets
+// `bad` where that does not hold: operands or a quotient that are not normal,
+// a Q at the bottom of a binade with a smaller quotient (the doubles below lie
+// closer).  A zero a is exact.
+__device__ __forceinline__ double quot64(double a, double b, uint64_t r, bool &bad) {
+    const uint32_t ah = hi64(a), al = lo64(a), bh = hi64(b), bl = lo64(b);
+    const uint32_t Ah = __funnelshift_l(al, (ah & 0xfffffu) | 0x100000u, 11), Al = al << 11;
+    const uint32_t rh = (uint32_t)(r >> 32), rl = (uint32_t)r;
+    const uint64_t m1 = (uint64_t)Ah * rl, m2 = (uint64_t)Al * rh;
+    uint64_t q = (uint64_t)Ah * rh + (m1 >> 32) + (m2 >> 32);  // A / B 2^62, within 9
+    const uint32_t ea = (ah >> 20) & 0x7ff, eb = (bh >> 20) & 0x7ff;
+    const bool up = (uint32_t)(q >> 32) >= 0x40000000u;  // A >= B
+    const uint32_t e = ea - eb + (up ? 1022 : 1021);     // biased exponent less one
+    if (!up) q += q;
+    q = (q + 512) >> 10;
+    const uint32_t Qh = (uint32_t)(q >> 32), Ql = (uint32_t)q, Bh = (bh & 0xfffffu) | 0x100000u;
+    // s is 52 or 53: the low word of A 2^s is zero, its high word A's low
+    // word shifted by s - 32
+    const uint64_t bq = (uint64_t)bl * Ql;
+    const uint32_t Rh = (al << (up ? 20 : 21)) - (uint32_t)(bq >> 32) - Bh * Ql - bl * Qh;
     const int64_t R = (int64_t)(((uint64_t)Rh << 32) - (uint32_t)bq);
     const int64_t B = (int64_t)(((uint64_t)Bh << 32) | bl);
-    const int64_t T = 2 * (R < 0 ? -R : R);
-    int k = (T > B ? 1 : 0) + (T > 3 * B ? 1 : 0);
-    if (R < 0) k = -k;
-    // q at the bottom of a binade with a smaller quotient (the doubles below lie
-    // closer), or carried two steps from the last of one (those above do not)
-    const bool edge = ((Qh == 0x100000u) & (ql < 4u) & (R < 0)) | ((Qh == 0x1fffffu) & (ql == ~0u) & (k == 2));
-    const bool range = (ea - 64u < 1919u) & (eq - 64u < 1919u);
-    bad |= (eb - 64u >= 1919u) | (!zero & (edge | !range));
-    if (zero) k = 0;
-    return __longlong_as_double(__double_as_longlong(q) + k);
+    const int k = (2 * R > B ? 1 : 0) - (2 * R < -B ? 1 : 0);
+    const bool zero = zero64(a);
+    bad |= (eb - 1u >= 2046u) |
+           (!zero & ((ea - 1u >= 2046u) | (e >= 2045u) | ((Qh == 0x100000u) & (Ql < 2u) & (R < 0))));
+    const uint64_t v = zero ? 0 : q + ((uint64_t)e << 52) + (int64_t)k;
+    return __longlong_as_double((long long)(v | ((uint64_t)((ah ^ bh) & 0x80000000u) << 32)));
 }
 
 // The operations of a cell.  mul: operands that may be zero; muln: operands
@@ -108,10 +119,8 @@ struct Fast64 {
     __device__ __forceinline__ double mul(double a, double b) { return mul64<true>(a, b, bad); }
     __device__ __forceinline__ double muln(double a, double b) { return mul64<false>(a, b, bad); }
     __device__ __forceinline__ double twice_plus(double a, double b) const { return __fma_rn(2.0, a, b); }
-    __device__ __forceinline__ double recip(double b) const { return recip64(b); }
-    __device__ __forceinline__ double quot(double a, double b, double y) {
-        return quot64(a, b, y, f.nzero, bad);
-    }
+    __device__ __forceinline__ uint64_t recip(double b) const { return recip64(b); }
+    __device__ __forceinline__ double quot(double a, double b, uint64_t r) { return quot64(a, b, r, bad); }
 };
 struct Plain64 {
     __device__ __forceinline__ double add(double a, double b) const { return a + b; }
@@ -119,8 +128,8 @@ struct Plain64 {
     __device__ __forceinline__ double mul(double a, double b) const { return a * b; }
     __device__ __forceinline__ double muln(double a, double b) const { return a * b; }
     __device__ __forceinline__ double twice_plus(double a, double b) const { return 2.0 * a + b; }
-    __device__ __forceinline__ double recip(double) const { return 0.0; }
-    __device__ __forceinline__ double quot(double a, double b, double) const { return a / b; }
+    __device__ __forceinline__ uint64_t recip(double) const { return 0; }
+    __device__ __forceinline__ double quot(double a, double b, uint64_t) const { return a / b; }
 };
 
 // x^m and x^n by repeated multiplication as power_broad does
@@ -194,9 +203,10 @@ template <class O>
 __device__ __forceinline__ void slip64(O &o, double h, double ux, double uy, double mu6, double delta6,
                                        double delta3sq, double &sx, double &sy) {
     const double den = o.add(o.twice_plus(o.muln(h, h), o.mul(delta6, h)), delta3sq);
-    const double mh = o.mul(mu6, h), y = o.recip(den);
-    sx = o.quot(o.mul(mh, ux), den, y);
-    sy = o.quot(o.mul(mh, uy), den, y);
+    const uint64_t r = o.recip(den);
+    const double mh = o.mul(mu6, h);
+    sx = o.quot(o.mul(mh, ux), den, r);
+    sy = o.quot(o.mul(mh, uy), den, r);
 }
 
 // equilibrium! (src/equilibrium.jl:67-114); g56 = 5/6 g, g15 = 1.5 g.  G0: no

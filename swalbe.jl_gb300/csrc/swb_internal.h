@@ -111,21 +111,19 @@ struct StepArgs {
     long long stop_at;
 };
 
-// Sums and products as fused multiply-adds: x * 1 + y rounds once, like x + y,
-// and x * y - 0 once, like x * y, signs of zero included.  On GB300 a stream of
-// DFMA with three register operands issues every 16.5 cycles per SM, one of
-// DADD or DMUL, or of DFMA with an operand from constant memory, every 19.1
-// (measured, 4 to 32 warps per SM).  So `one` and `nzero` (1 and -0) are kernel
-// arguments moved to registers by in_registers(): of constants the compiler
-// would make sums and products again.
+// Sums as fused multiply-adds: x * 1 + y rounds once, like x + y, signs of zero
+// included.  On GB300 a stream of DFMA with three register operands issues every
+// 16.5 cycles per SM, one of DADD or DMUL, or of DFMA with an operand from
+// constant memory, every 19.1 (measured, 4 to 32 warps per SM).  So `one` (1) is
+// a kernel argument moved to a register by in_registers(): of a constant the
+// compiler would make sums again.
 struct Fma64 {
-    double one, nzero;
+    double one;
     __device__ __forceinline__ double add(double a, double b) const { return __fma_rn(a, one, b); }
     __device__ __forceinline__ double sub(double a, double b) const { return __fma_rn(-b, one, a); }
-    __device__ __forceinline__ double mul(double a, double b) const { return __fma_rn(a, b, nzero); }
     __device__ __forceinline__ Fma64 in_registers() const {
         Fma64 f = *this;
-        asm volatile("" : "+d"(f.one), "+d"(f.nzero));
+        asm volatile("" : "+d"(f.one));
         return f;
     }
 };

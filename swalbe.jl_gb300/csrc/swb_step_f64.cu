@@ -39,7 +39,8 @@ namespace swb {
 // (302 Float64 instructions per cell; here 145, and with the products in
 // integers 94): 600 iterations of a 256² droplet 41.1 -> 16.0 -> 12.6 ms, 60 of a
 // 1000 x 1030 film 34.3 -> 17.1 -> 13.2 ms (upload and download included), 512²
-// 141 -> 77 -> 57 us per iteration.  A 56 x 40 film, one warp per SM quarter, is
+// 141 -> 77 -> 57 us per iteration; with the reciprocals in integers as well
+// (80 instructions) 52 us, and 1000 x 1030 195 -> 181.  A 56 x 40 film, one warp per SM quarter, is
 // bound by latency: 43.7 -> 10.7 -> 11.1 us.  (One kernel of 8 x 4 tiles with
 // recomputed halos: 9.4 there, but 12.4 at 128 x 96 and 104 at 512².)
 constexpr int kCellNT = 128;
@@ -304,11 +305,11 @@ __device__ __forceinline__ void cell_area(const StepArgs &a, const Cell64 &x, co
     }
 }
 
-// Six blocks per SM (80 registers, 36 bytes of spill) instead of the four that
-// the compiler's 106 registers leave: 256² 24.9 -> 19.9 us per iteration, 301 x
-// 257 30.6 -> 20.8, 1000 x 1030 208 -> 195.
+// Seven blocks per SM (72 registers, a little spill) instead of the four that the
+// compiler's 106 registers leave: with six, 256² 24.9 -> 19.9 us per iteration and
+// 1000 x 1030 208 -> 195; seven against six, 1000 x 1030 183 -> 181.
 template <bool TAU1, bool G0, bool GEN>
-__global__ void __launch_bounds__(kCellNT, 6) cell_collide_kernel(const __grid_constant__ StepArgs a,
+__global__ void __launch_bounds__(kCellNT, 7) cell_collide_kernel(const __grid_constant__ StepArgs a,
                                                                const __grid_constant__ Cell64 x, int k) {
     const int c = blockIdx.x * kCellNT + threadIdx.x, N = a.Lx * a.Ly;
     const int cc = c < N ? c : 0;
@@ -345,9 +346,9 @@ __device__ __noinline__ void cell_velocity_again(double h, double jx, double jy,
 __device__ __forceinline__ void cell_velocity(const Cell64 &x, double h, double jx, double jy, double &ux,
                                               double &uy) {
     Fast64 o(x.f);
-    const double y = o.recip(h);
-    ux = o.quot(jx, h, y);
-    uy = o.quot(jy, h, y);
+    const uint64_t r = o.recip(h);
+    ux = o.quot(jx, h, r);
+    uy = o.quot(jy, h, r);
     if (o.bad) {
         double vx, vy;
         cell_velocity_again(h, jx, jy, &vx, &vy);
@@ -797,10 +798,10 @@ __global__ void k_moments(PlainState s, Fma64 g) {
         plain_cell<3>(g, [=](auto &o, double *q) {
             double h, jx, jy;
             moments64(o, v.f, h, jx, jy);
-            const double y = o.recip(h);
+            const uint64_t r = o.recip(h);
             q[0] = h;
-            q[1] = o.quot(jx, h, y);
-            q[2] = o.quot(jy, h, y);
+            q[1] = o.quot(jx, h, r);
+            q[2] = o.quot(jy, h, r);
         }, r);
         s.h[c] = r[0];
         s.ux[c] = r[1];
@@ -816,7 +817,7 @@ constexpr int kPlainNT = 64;
 #define PLAIN_LAUNCH(kernel, s, st, ...)                                                               \
     do {                                                                                               \
         count_launches(1);                                                                             \
-        return launch_step(kernel, grid_for((s).N, kPlainNT), kPlainNT, st, s, Fma64{1.0, -0.0}, ##__VA_ARGS__); \
+        return launch_step(kernel, grid_for((s).N, kPlainNT), kPlainNT, st, s, Fma64{1.0}, ##__VA_ARGS__); \
     } while (0)
 
 cudaError_t plain_filmpressure(const PlainState &s, const double *kapF, double kap, double gamma,
@@ -846,7 +847,7 @@ cudaError_t plain_equilibrium(const PlainState &s, double g, cudaStream_t st) {
 cudaError_t plain_bgk_stream(PlainState &s, double omeg, double invtau, cudaStream_t st) {
     count_launches(1);
     const cudaError_t e = launch_step(k_bgk_stream, grid_for(s.N, kPlainNT), kPlainNT, st, s,
-                                      Fma64{1.0, -0.0}, omeg, invtau);
+                                      Fma64{1.0}, omeg, invtau);
     if (e == cudaSuccess) {
         double *f = s.fout;
         s.fout = s.ftemp;
