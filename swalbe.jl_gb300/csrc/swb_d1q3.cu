@@ -67,6 +67,18 @@ struct D1Part {
 
 namespace {
 
+// A cell's constants, and its slippage and equilibrium.
+template <class R>
+struct D1Cell {
+    R kap, gam, dg;  // κ, surface tension and ∇γ of the cell
+    R mu6, delta6, delta3sq, omeg, invtau, g, g25, g50;
+    bool grad, tau1;
+};
+template <class R>
+struct D1Mid {
+    R slip, fe[3];
+};
+
 // One cell's operations, Float64: rounded as the reference's, with products by
 // powers of two inside the sum that follows them (exact, short of subnormal
 // numbers).
@@ -74,31 +86,31 @@ template <class O>
 struct D1Cell64 {
     O o;
     __device__ __forceinline__ double quot(double a, double b) { return o.quot(a, b, o.recip(b)); }
-    __device__ __forceinline__ double pressure(const D1Args &a, double h, double hip, double him, double kap,
-                                               double gam) {
+    __device__ __forceinline__ double pressure(const D1Args &a, const D1Cell<double> &c, double h, double hip,
+                                               double him) {
         double pn, pm;
         powers64(o, quot(a.hmin, o.add(h, a.hcrit)), a.n, a.m, pn, pm);
-        const double p = o.mul(-gam, o.mul(kap, o.sub(pn, pm)));
-        return o.sub(p, o.mul(gam, o.add(o.twice_plus(-h, hip), him)));
+        const double p = o.mul(-c.gam, o.mul(c.kap, o.sub(pn, pm)));
+        return o.sub(p, o.mul(c.gam, o.add(o.twice_plus(-h, hip), him)));
     }
-    __device__ __forceinline__ double force(double h, double u, double pm, double pp, double mu6,
-                                            double delta6, double delta3sq) {
-        const double den = o.add(o.twice_plus(o.muln(h, h), o.mul(delta6, h)), delta3sq);
-        const double slip = quot(o.mul(o.mul(mu6, h), u), den);
-        return __fma_rn(0.5, o.mul(h, o.sub(pm, pp)), -slip);
-    }
-    __device__ __forceinline__ double sub(double a, double b) { return o.sub(a, b); }
-    __device__ __forceinline__ void collide(double h, double u, double F, double g, double omeg, double invtau,
-                                            bool tau1, const double fo[3], double out[3]) {
+    // slippage and equilibrium, which need only the cell's own fields
+    __device__ __forceinline__ void local(const D1Cell<double> &c, double h, double u, D1Mid<double> &m) {
+        const double den = o.add(o.twice_plus(o.muln(h, h), o.mul(c.delta6, h)), c.delta3sq);
+        m.slip = quot(o.mul(o.mul(c.mu6, h), u), den);
         const double uu = o.mul(u, u);
-        double fe[3];
-        const double gh = g == 0.0 ? 0.0 : o.muln(0.25 * g, h);
-        fe[0] = o.muln(h, o.sub(g == 0.0 ? 1.0 : o.sub(1.0, o.muln(0.5 * g, h)), uu));
-        fe[1] = o.mul(h, __fma_rn(0.5, uu, __fma_rn(0.5, u, gh)));
-        fe[2] = o.mul(h, __fma_rn(0.5, uu, __fma_rn(-0.5, u, gh)));
-        if (!tau1)
+        const double gh = c.g == 0.0 ? 0.0 : o.muln(c.g25, h);
+        m.fe[0] = o.muln(h, o.sub(c.g == 0.0 ? 1.0 : o.sub(1.0, o.muln(c.g50, h)), uu));
+        m.fe[1] = o.mul(h, __fma_rn(0.5, uu, __fma_rn(0.5, u, gh)));
+        m.fe[2] = o.mul(h, __fma_rn(0.5, uu, __fma_rn(-0.5, u, gh)));
+    }
+    __device__ __forceinline__ void second(const D1Cell<double> &c, double h, const D1Mid<double> &m, double pm,
+                                           double pp, const double fo[3], double out[3]) {
+        double F = __fma_rn(0.5, o.mul(h, o.sub(pm, pp)), -m.slip);
+        if (c.grad) F = o.sub(F, c.dg);
+        double fe[3] = {m.fe[0], m.fe[1], m.fe[2]};
+        if (!c.tau1)
 #pragma unroll
-            for (int q = 0; q < 3; ++q) fe[q] = o.add(o.mul(omeg, fo[q]), o.mul(invtau, fe[q]));
+            for (int q = 0; q < 3; ++q) fe[q] = o.add(o.mul(c.omeg, fo[q]), o.mul(c.invtau, fe[q]));
         out[0] = fe[0];
         out[1] = __fma_rn(0.5, F, fe[1]);
         out[2] = __fma_rn(-0.5, F, fe[2]);
@@ -108,54 +120,60 @@ struct D1Cell64 {
         u = quot(o.sub(f[1], f[2]), h);
     }
 };
-// The three parts of an iteration with the integer unit's help, each computed
-// again out of line where that met a number it does not hold.
-__device__ __noinline__ double d1_pressure_again(const D1Args &a, double h, double hip, double him, double kap,
-                                                 double gam) {
-    return D1Cell64<Plain64>{}.pressure(a, h, hip, him, kap, gam);
+// The parts of an iteration with the integer unit's help, each computed again
+// out of line where that met a number it does not hold.
+__device__ __noinline__ double d1_pressure_again(const D1Args &a, const D1Cell<double> &c, double h, double hip,
+                                                 double him) {
+    return D1Cell64<Plain64>{}.pressure(a, c, h, hip, him);
 }
-__device__ __noinline__ double d1_force_again(double h, double u, double pm, double pp, double mu6,
-                                              double delta6, double delta3sq) {
-    return D1Cell64<Plain64>{}.force(h, u, pm, pp, mu6, delta6, delta3sq);
+__device__ __noinline__ void d1_local_again(const D1Cell<double> &c, double h, double u, D1Mid<double> *m) {
+    D1Cell64<Plain64>{}.local(c, h, u, *m);
 }
-__device__ __noinline__ void d1_collide_again(double h, double u, double F, double g, double omeg,
-                                              double invtau, bool tau1, const double *fo, double *out) {
-    D1Cell64<Plain64>{}.collide(h, u, F, g, omeg, invtau, tau1, fo, out);
+__device__ __noinline__ void d1_second_again(const D1Cell<double> &c, double h, const D1Mid<double> &m, double pm,
+                                             double pp, const double *fo, double *out) {
+    D1Cell64<Plain64>{}.second(c, h, m, pm, pp, fo, out);
 }
 __device__ __noinline__ void d1_moments_again(const double *f, double *h, double *u) {
     D1Cell64<Plain64>{}.moments(f, *h, *u);
 }
 struct D1Ops64 {
     Fma64 f;
-    __device__ __forceinline__ double pressure(const D1Args &a, double h, double hip, double him, double kap,
-                                               double gam) const {
-        D1Cell64<Fast64> c{Fast64(f)};
-        const double p = c.pressure(a, h, hip, him, kap, gam);
-        return c.o.bad ? d1_pressure_again(a, h, hip, him, kap, gam) : p;
+    __device__ __forceinline__ double pressure(const D1Args &a, const D1Cell<double> &c, double h, double hip,
+                                               double him) const {
+        D1Cell64<Fast64> k{Fast64(f)};
+        const double p = k.pressure(a, c, h, hip, him);
+        if (!k.o.bad) return p;
+        const D1Cell<double> cc = c;
+        return d1_pressure_again(a, cc, h, hip, him);
     }
-    __device__ __forceinline__ double force(double h, double u, double pm, double pp, double mu6,
-                                            double delta6, double delta3sq) const {
-        D1Cell64<Fast64> c{Fast64(f)};
-        const double F = c.force(h, u, pm, pp, mu6, delta6, delta3sq);
-        return c.o.bad ? d1_force_again(h, u, pm, pp, mu6, delta6, delta3sq) : F;
+    __device__ __forceinline__ void local(const D1Cell<double> &c, double h, double u, D1Mid<double> &m) const {
+        D1Cell64<Fast64> k{Fast64(f)};
+        k.local(c, h, u, m);
+        if (k.o.bad) {
+            const D1Cell<double> cc = c;
+            D1Mid<double> again;
+            d1_local_again(cc, h, u, &again);
+            m = again;
+        }
     }
-    __device__ __forceinline__ double sub(double a, double b) const { return f.sub(a, b); }
-    __device__ __forceinline__ void collide(double h, double u, double F, double g, double omeg, double invtau,
-                                            bool tau1, const double fo[3], double out[3]) const {
-        D1Cell64<Fast64> c{Fast64(f)};
-        c.collide(h, u, F, g, omeg, invtau, tau1, fo, out);
-        if (c.o.bad) {
+    __device__ __forceinline__ void second(const D1Cell<double> &c, double h, const D1Mid<double> &m, double pm,
+                                           double pp, const double fo[3], double out[3]) const {
+        D1Cell64<Fast64> k{Fast64(f)};
+        k.second(c, h, m, pm, pp, fo, out);
+        if (k.o.bad) {
+            const D1Cell<double> cc = c;
+            const D1Mid<double> mm = m;
             const double in[3] = {fo[0], fo[1], fo[2]};
             double again[3];
-            d1_collide_again(h, u, F, g, omeg, invtau, tau1, in, again);
+            d1_second_again(cc, h, mm, pm, pp, in, again);
 #pragma unroll
             for (int q = 0; q < 3; ++q) out[q] = again[q];
         }
     }
     __device__ __forceinline__ void moments(const double fo[3], double &h, double &u) const {
-        D1Cell64<Fast64> c{Fast64(f)};
-        c.moments(fo, h, u);
-        if (c.o.bad) {
+        D1Cell64<Fast64> k{Fast64(f)};
+        k.moments(fo, h, u);
+        if (k.o.bad) {
             const double in[3] = {fo[0], fo[1], fo[2]};
             double ha, ua;
             d1_moments_again(in, &ha, &ua);
@@ -173,27 +191,27 @@ struct D1Ops32 {
         for (int i = 0; i < n; ++i) t *= x;
         return t;
     }
-    __device__ __forceinline__ float pressure(const D1Args &a, float h, float hip, float him, float kap,
-                                              float gam) const {
+    __device__ __forceinline__ float pressure(const D1Args &a, const D1Cell<float> &c, float h, float hip,
+                                              float him) const {
         const float x = float(a.hmin) / (h + float(a.hcrit));
-        const float p = -gam * (kap * (pow_n(x, a.n) - pow_n(x, a.m)));
-        return p - gam * ((hip - 2.0f * h) + him);
+        const float p = -c.gam * (c.kap * (pow_n(x, a.n) - pow_n(x, a.m)));
+        return p - c.gam * ((hip - 2.0f * h) + him);
     }
-    __device__ __forceinline__ float force(float h, float u, float pm, float pp, float mu6, float delta6,
-                                           float delta3sq) const {
-        const float hgp = (h * -0.5f) * (pm - pp);
-        return -hgp - (mu6 * h * u) / ((2.0f * (h * h) + delta6 * h) + delta3sq);
-    }
-    __device__ __forceinline__ float sub(float a, float b) const { return a - b; }
-    __device__ __forceinline__ void collide(float h, float u, float F, float g, float omeg, float invtau, bool,
-                                            const float fo[3], float o[3]) const {
+    __device__ __forceinline__ void local(const D1Cell<float> &c, float h, float u, D1Mid<float> &m) const {
+        m.slip = (c.mu6 * h * u) / ((2.0f * (h * h) + c.delta6 * h) + c.delta3sq);
         const float uu = u * u;
-        const float fe0 = h * ((1.0f - (0.5f * g) * h) - uu);
-        const float fe1 = h * (((0.25f * g) * h + 0.5f * u) + 0.5f * uu);
-        const float fe2 = h * (((0.25f * g) * h - 0.5f * u) + 0.5f * uu);
-        o[0] = omeg * fo[0] + invtau * fe0;
-        o[1] = omeg * fo[1] + invtau * fe1 + 0.5f * F;
-        o[2] = omeg * fo[2] + invtau * fe2 - 0.5f * F;
+        m.fe[0] = h * ((1.0f - (0.5f * c.g) * h) - uu);
+        m.fe[1] = h * (((0.25f * c.g) * h + 0.5f * u) + 0.5f * uu);
+        m.fe[2] = h * (((0.25f * c.g) * h - 0.5f * u) + 0.5f * uu);
+    }
+    __device__ __forceinline__ void second(const D1Cell<float> &c, float h, const D1Mid<float> &m, float pm,
+                                           float pp, const float fo[3], float out[3]) const {
+        const float hgp = (h * -0.5f) * (pm - pp);
+        float F = -hgp - m.slip;
+        if (c.grad) F = F - c.dg;
+        out[0] = c.omeg * fo[0] + c.invtau * m.fe[0];
+        out[1] = c.omeg * fo[1] + c.invtau * m.fe[1] + 0.5f * F;
+        out[2] = c.omeg * fo[2] + c.invtau * m.fe[2] - 0.5f * F;
     }
     __device__ __forceinline__ void moments(const float o[3], float &h, float &u) const {
         h = (o[0] + o[1]) + o[2];
@@ -234,8 +252,14 @@ __device__ __forceinline__ void d1_measure(D1Part *out, bool own, double h, bool
 
 // n iterations of the cells of chunk blockIdx.x, from the buffers `from` to the
 // others.  part: this launch's measures, [n][gridDim.x][kD1NT / 32] (or null).
+// Float64 has two threads per cell: the first kD1NT compute pressures (and the
+// measures) while the others compute slippage and equilibrium, the two long
+// chains of an iteration, and then collide and stream (2.82 -> 2.58 us per
+// iteration; FP32, whose chains are short, 0.94 -> 0.97 and so one thread).
+template <class R>
+constexpr int kD1Halves = sizeof(R) == 8 ? 2 : 1;
 template <class R, class Ops>
-__global__ void __launch_bounds__(kD1NT) d1q3_run_kernel(const D1Args *__restrict__ args,
+__global__ void __launch_bounds__(kD1Halves<R> * kD1NT) d1q3_run_kernel(const D1Args *__restrict__ args,
                                                          const D1Chunk *__restrict__ table, const Ops op,
                                                          int from, int n, D1Part *part) {
     __shared__ D1Args a;
@@ -245,7 +269,9 @@ __global__ void __launch_bounds__(kD1NT) d1q3_run_kernel(const D1Args *__restric
     __syncthreads();
     grid_dep_wait();
     grid_dep_launch();
-    const int t = threadIdx.x, L = a.L;
+    const int t = threadIdx.x & (kD1NT - 1), L = a.L;
+    const bool first = threadIdx.x < kD1NT;  // computes pressures (whole warps)
+    const bool second = kD1Halves<R> == 1 || !first;  // holds the cell's state
     const bool whole = ck.w == L && L <= kD1NT;  // periodic within the CTA
     const int halo = whole ? 0 : 3 * n, span = ck.w + 2 * halo;
     const bool in = t < span, own = t >= halo && t < halo + ck.w;
@@ -255,39 +281,52 @@ __global__ void __launch_bounds__(kD1NT) d1q3_run_kernel(const D1Args *__restric
     // neighbours; at the ends of a span with halos their values do not matter
     const int tm = t == 0 ? (whole ? span - 1 : 0) : t - 1;
     const int tp = t >= span - 1 ? (whole ? 0 : span - 1) : t + 1;
-    const R mu6 = R(6) * R(a.mu), delta6 = R(6) * R(a.delta), delta3sq = R(3) * (R(a.delta) * R(a.delta));
-    const R omeg = R(a.omeg), invtau = R(a.invtau), grav = R(a.g);
-    const bool tau1 = a.omeg == 0.0 && a.invtau == 1.0;
-    const R kap = a.kapF ? reinterpret_cast<const R *>(a.kapF)[g] : R(a.kap);
-    const R gam = a.gamF ? reinterpret_cast<const R *>(a.gamF)[g] : R(a.gamma);
-    const R dg = a.dgF ? reinterpret_cast<const R *>(a.dgF)[g] : R(0);
-    const bool grad = a.dgF != nullptr, rec = part != nullptr && a.rec;
+    D1Cell<R> c;
+    c.mu6 = R(6) * R(a.mu);
+    c.delta6 = R(6) * R(a.delta);
+    c.delta3sq = R(3) * (R(a.delta) * R(a.delta));
+    c.omeg = R(a.omeg);
+    c.invtau = R(a.invtau);
+    c.tau1 = a.omeg == 0.0 && a.invtau == 1.0;
+    c.g = R(a.g);
+    c.g25 = R(0.25) * c.g;
+    c.g50 = R(0.5) * c.g;
+    c.kap = a.kapF ? reinterpret_cast<const R *>(a.kapF)[g] : R(a.kap);
+    c.gam = a.gamF ? reinterpret_cast<const R *>(a.gamF)[g] : R(a.gamma);
+    c.dg = a.dgF ? reinterpret_cast<const R *>(a.dgF)[g] : R(0);
+    c.grad = a.dgF != nullptr;
+    const bool rec = part != nullptr && a.rec;
     const R *ff = reinterpret_cast<const R *>(a.f[from]);
     R h = reinterpret_cast<const R *>(a.h[from])[g], u = reinterpret_cast<const R *>(a.u[from])[g];
     R fo[3] = {ff[g], ff[L + g], ff[2 * L + g]}, p = R(0);
     int bad = 0;
 #pragma unroll 1
     for (int k = 0; k < n; ++k) {
-        sh[t] = h;
+        if (second) sh[t] = h;
         __syncthreads();
-        if (rec)
-            d1_measure(part + ((size_t)k * gridDim.x + blockIdx.x) * (kD1NT / 32) + (t >> 5), own, (double)h,
-                       h > R(0.055));
-        if (in) {
-            p = op.pressure(a, h, sh[tm], sh[tp], kap, gam);
-            sp[t] = p;
+        D1Mid<R> m;
+        if (first) {
+            const R hc = sh[t];
+            if (in) {
+                p = op.pressure(a, c, hc, sh[tm], sh[tp]);
+                sp[t] = p;
+            }
+            if (rec)
+                d1_measure(part + ((size_t)k * gridDim.x + blockIdx.x) * (kD1NT / 32) + (t >> 5), own, (double)hc,
+                           hc > R(0.055));
+        }
+        if (second && in) {
+            op.local(c, h, u, m);
         }
         __syncthreads();
         R o[3];
-        if (in) {
-            R F = op.force(h, u, sp[tm], sp[tp], mu6, delta6, delta3sq);
-            if (grad) F = op.sub(F, dg);
-            op.collide(h, u, F, grav, omeg, invtau, tau1, fo, o);
+        if (second && in) {
+            op.second(c, h, m, sp[tm], sp[tp], fo, o);
             s1[t] = o[1];
             s2[t] = o[2];
         }
         __syncthreads();
-        if (in) {
+        if (second && in) {
             fo[0] = o[0];
             fo[1] = s1[tm];
             fo[2] = s2[tp];
@@ -295,15 +334,15 @@ __global__ void __launch_bounds__(kD1NT) d1q3_run_kernel(const D1Args *__restric
             if (own && !finite(h)) bad = 1;
         }
     }
-    if (own) {
-        R *fn = reinterpret_cast<R *>(a.f[from ^ 1]);
-        reinterpret_cast<R *>(a.h[from ^ 1])[g] = h;
-        reinterpret_cast<R *>(a.u[from ^ 1])[g] = u;
-        reinterpret_cast<R *>(a.p)[g] = p;
+    if (!own) return;
+    if (first) reinterpret_cast<R *>(a.p)[g] = p;
+    if (!second) return;
+    R *fn = reinterpret_cast<R *>(a.f[from ^ 1]);
+    reinterpret_cast<R *>(a.h[from ^ 1])[g] = h;
+    reinterpret_cast<R *>(a.u[from ^ 1])[g] = u;
 #pragma unroll
-        for (int q = 0; q < 3; ++q) fn[q * L + g] = fo[q];
-        if (bad) *a.nan_flag = 1;
-    }
+    for (int q = 0; q < 3; ++q) fn[q * L + g] = fo[q];
+    if (bad) *a.nan_flag = 1;
 }
 
 // The records of n iterations after t0 from their warps' measures: one warp
@@ -698,11 +737,13 @@ int swb1d_step(swb1d *b, int64_t nsteps) {
             swb::D1Part *part =
                 b->rec_cap ? b->d_part + (size_t)done * b->nchunks * (swb::kD1NT / 32) : nullptr;
             const swb::Fma64 f{1.0};
+            auto run = [&](auto *kern, int halves, auto ops) {
+                return swb::launch_step(kern, b->nchunks, halves * swb::kD1NT, b->stream, b->d_args, b->d_chunks, ops,
+                                        b->cur, n, part);
+            };
             const cudaError_t e =
-                b->rb == 8 ? swb::launch_step(swb::d1q3_run_kernel<double, swb::D1Ops64>, b->nchunks, swb::kD1NT,
-                                              b->stream, b->d_args, b->d_chunks, swb::D1Ops64{f}, b->cur, n, part)
-                           : swb::launch_step(swb::d1q3_run_kernel<float, swb::D1Ops32>, b->nchunks, swb::kD1NT,
-                                              b->stream, b->d_args, b->d_chunks, swb::D1Ops32{f}, b->cur, n, part);
+                b->rb == 8 ? run(swb::d1q3_run_kernel<double, swb::D1Ops64>, swb::kD1Halves<double>, swb::D1Ops64{f})
+                           : run(swb::d1q3_run_kernel<float, swb::D1Ops32>, swb::kD1Halves<float>, swb::D1Ops32{f});
             D1_TRY(b, e);
             swb::count_launches(1);
             b->cur ^= 1;
