@@ -337,6 +337,7 @@ struct swb_state {
     cudaGraphExec_t gexec = nullptr;
     int gsteps = 0;
     bool gvalid = false;
+    long long direct = 0;  // Float64: iterations launched one by one so far
     double *dtmp = nullptr;
     size_t dtmp_bytes = 0;
     // snapshots: device ring of snap_cap heights taken every snap_every iterations
@@ -531,6 +532,13 @@ int plain_iteration(swb_state *s) {
 }
 
 constexpr int kGraphSteps = 64;
+// A Float64 state's first iterations are launched one by one: they are three
+// kernels that take the GPU longer (11 us on the smallest lattices) than the
+// host needs to launch them (5 us), and a graph of 64 takes 0.5 ms to build
+// (200 iterations of a 56 x 40 film, state and results included: 3.55 ms with
+// a graph, 3.26 without).  Graphs of 16 build faster, but every one costs a
+// pause: 11.1 -> 11.9 us per iteration.
+constexpr long long kCellGraphMin = 512;
 
 // Geometries chosen by the autotuner, per (Lx, Ly, precision), process-wide.
 std::mutex g_tune_mu;
@@ -817,7 +825,8 @@ int fused_steps(swb_state *s, long long nsteps) {
         if (left > 0) CUDA_TRY(&s->err, run_sequence(s, left));
         left = 0;
     }
-    if (left >= kGraphSteps) {
+    if (cells) s->direct += left;
+    if (left >= kGraphSteps && (!cells || s->gvalid || s->direct >= kCellGraphMin)) {
         if (!s->gvalid) {
             cudaGraph_t g = nullptr;
             CUDA_TRY(&s->err, cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
