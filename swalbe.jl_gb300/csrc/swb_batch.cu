@@ -7,6 +7,7 @@
 #include <array>
 #include <chrono>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "swb_lattice.h"
@@ -251,13 +252,14 @@ int upload_args(swb_batch *b) {
 }
 
 // Strip geometry of every lattice (nt < 0: pair strips, which need FP32
-// arithmetic and even Lx everywhere) and the tile tables.
-int apply_geometry(swb_batch *b, int nt, int rows) {
+// arithmetic and even Lx everywhere), of `rows` rows or (balanced) of at most
+// that many with the lattice's strips equally high, and the tile tables.
+int apply_geometry(swb_batch *b, int nt, int rows, bool balanced) {
     B_TRY(b, cudaStreamSynchronize(b->stream));
     b->nt = nt;
     b->rows = rows;
     for (int i = 0; i < b->count; ++i) {
-        int h = rows < b->params[i].Ly ? rows : b->params[i].Ly;
+        int h = balanced ? swb::balanced_rows(b->params[i].Ly, rows) : std::min(rows, b->params[i].Ly);
         if (h < swb::kMinRows) h = swb::kMinRows;
         swb::set_geometry(b->args[i], nt, h);
     }
@@ -331,15 +333,32 @@ int autotune(swb_batch *b, long long &left) {
         pair = pair && swb::pair_form_ok(a);
         wave = wave || a.theta_mode == swb::THETA_WAVE;
     }
-    std::vector<std::array<int, 2>> geos = {{64, 32}, {64, 16}, {128, 16}};
-    if (pair_possible(b) && pair) {
-        geos.push_back({-64, 16});
-        geos.push_back({-64, 32});
-        geos.push_back({-64, 64});
-        geos.push_back({-32, 16});
+    std::vector<std::array<int, 2>> geos;
+    if (b->geometry_fixed) {  // a geometry set by the caller
+        geos = {{b->nt, b->rows}};
+    } else {
+        // the four pair geometries with the shortest estimates, of different
+        // numbers of strips, then one-column strips
+        if (pair_possible(b) && pair) {
+            std::vector<std::pair<int, int>> sizes;
+            for (const swb_params &p : b->params) sizes.push_back({p.Lx, p.Ly});
+            std::vector<std::tuple<double, int, int>> est;
+            for (int nt : {-64, -32}) {
+                const int slots = swb::batch_blocks_per_sm(b->precision, nt, wave);
+                double last = -1.0;
+                for (int cap = 64; cap >= swb::kMinRows; --cap) {
+                    const double us = swb::pair_iteration_us(sizes, nt, cap, sms, slots);
+                    if (us != last) est.push_back({us, nt, cap});
+                    last = us;
+                }
+            }
+            std::sort(est.begin(), est.end());
+            for (size_t i = 0; i < est.size() && i < 4; ++i) geos.push_back({std::get<1>(est[i]), std::get<2>(est[i])});
+        }
+        geos.push_back({64, 32});
+        geos.push_back({64, 16});
     }
-    if (b->geometry_fixed) geos = {{b->nt, b->rows}};  // a geometry set by the caller
-    const int probe = 2;
+    const int probe = 4;
     struct Best {
         float ms = 1e30f;
         int nt = 0, rows = 0, grid = 0;
@@ -351,7 +370,7 @@ int autotune(swb_batch *b, long long &left) {
     for (auto &g : geos) {
         if (rc) break;
         if (g[0] != b->nt || g[1] != b->rows) {
-            rc = apply_geometry(b, g[0], g[1]);
+            rc = apply_geometry(b, g[0], g[1], !b->geometry_fixed);
             if (rc) break;
         }
         const int occ = swb::batch_blocks_per_sm(b->precision, b->nt, wave);
@@ -379,13 +398,13 @@ int autotune(swb_batch *b, long long &left) {
     if (rc) return rc;
     if (best.nt == 0) {  // too few steps to probe: the default strips, persistent CTAs
         if (b->nt != swb::kBatchNT || b->rows != swb::kBatchRows) {
-            rc = apply_geometry(b, swb::kBatchNT, swb::kBatchRows);
+            rc = apply_geometry(b, swb::kBatchNT, swb::kBatchRows, false);
             if (rc) return rc;
         }
         b->grid = std::min(b->ntiles, sms * swb::batch_blocks_per_sm(b->precision, b->nt, wave));
     } else {
         if (best.nt != b->nt || best.rows != b->rows) {
-            rc = apply_geometry(b, best.nt, best.rows);
+            rc = apply_geometry(b, best.nt, best.rows, !b->geometry_fixed);
             if (rc) return rc;
         }
         b->grid = best.grid;
@@ -568,7 +587,7 @@ int swb_batch_set_geometry(swb_batch *b, int nt, int rows) {
     if (nt < 0 && !pair_possible(b))
         return swb::bfail(&b->err, SWB_ERR_UNSUPPORTED,
                           "batch pair strips: FP32 or FP16 storage and even Lx in every lattice");
-    const int rc = apply_geometry(b, nt, rows);
+    const int rc = apply_geometry(b, nt, rows, false);
     if (rc) return rc;
     b->geometry_fixed = true;
     b->tuned = false;  // re-pick the CTA count (the tuner keeps this geometry)

@@ -5,6 +5,7 @@
 
 #include <cmath>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "swb_internal.h"
@@ -52,6 +53,35 @@ inline LatticeLayout lattice_layout(const swb_params &p, int precision) {
 // its many lattices, so strips can be tall (fewer halo rows re-pulled; on
 // GB300 the ensemble ran 26 GLUPS at 124x4 strips, 45 GLUPS at 60x32).
 constexpr int kBatchRows = 32;
+
+// Rows of the strips that cover Ly rows with as few strips of at most `cap` rows
+// as that takes, all about equally high.
+inline int balanced_rows(int Ly, int cap) {
+    const int strips = (Ly + cap - 1) / cap;
+    return (Ly + strips - 1) / strips;
+}
+// Estimated time of an iteration of many lattices (Lx, Ly) on pair strips of
+// geometry nt and at most cap rows, balanced: launch and drain, then waves of
+// up to `slots` CTAs per SM, each as long as a march over the tallest strip.
+// c CTAs of 64 threads (or 2 c of 32) on an SM take 0.655 us per row up to
+// c = 1.4 and 0.11 us more for each further one.  Measured on GB300 with the θ
+// wave: 64 to 4M cells in 1 to 32 lattices, 18 geometries each; the estimate is
+// within 20 % of all, and the strips it picks within 15 % of the best.  E.g. a
+// 1024² lattice 50.7 us with 64 rows, 21.0 with 8; eight of 32k to 147k cells
+// 51.1 and 17.7 (60 columns, 6 rows).
+inline double pair_iteration_us(const std::vector<std::pair<int, int>> &sizes, int nt, int cap, int sms, int slots) {
+    const int w = -2 * nt - 4;
+    double strips = 0.0;
+    int tallest = 0;
+    for (const auto &p : sizes) {
+        const int h = balanced_rows(p.second, cap);
+        tallest = h > tallest ? h : tallest;
+        strips += (double)((p.first + w - 1) / w) * (double)((p.second + h - 1) / h);
+    }
+    const double c = strips / sms, waves = std::floor(c / slots), rest = c - slots * waves;
+    auto row = [nt](double c) { return 0.655 * (1.0 + 0.17 * std::fmax(0.0, c * (-nt / 64.0) - 1.4)); };
+    return 4.7 + (tallest + 4) * (waves * row(slots) + (rest > 0.0 ? row(rest) : 0.0));
+}
 
 // Step arguments of a lattice whose buffers start at `base`; strips of
 // nt threads and `rows` rows (capped at the lattice height).

@@ -185,50 +185,38 @@ bool admit_device(swb_server *sv, Req *r) {
 // fill the GPU takes short strips although they recompute more.  Results do
 // not depend on the geometry.
 constexpr int kServePairRows = 64;
-int balanced_rows(int Ly, int cap) {
-    const int strips = (Ly + cap - 1) / cap;
-    return (Ly + strips - 1) / strips;
-}
-// Estimated time of an iteration with strips of geometry nt and at most cap
-// rows.  Pair strips: launch and drain, then waves of up to 8 CTAs of 64
-// threads (16 of 32) per SM, each as long as a march over the tallest strip,
-// whose rows take 0.655 us alone on an SM and 2.1 times that in a full wave
-// (measured on GB300: 64 to 4M cells in 1 to 32 lattices, 18 geometries each;
-// the estimate is within 20 % of all, and the one it picks within 15 % of the
-// best).  E.g. a 1024² lattice 50.7 us with 64 rows, 21.0 with 8; eight of 32k
-// to 147k cells 51.1 and 17.7 (60 columns, 6 rows).  One-column strips: the
-// march at 0.6 us per row (Float64: 10) or 55 cells per ns (2).
-double iteration_us(const swb_server *sv, int nt, int cap, int sms) {
-    const int w = nt < 0 ? -2 * nt - 4 : nt - 4;
-    double strips = 0.0, cells = 0.0;
+// Estimated time of an iteration of the resident set.  Pair strips:
+// pair_iteration_us.  One-column strips: the march of the tallest at 0.6 us per
+// row (Float64: 10), or 55 cells per ns (2).
+double iteration_us(const swb_server *sv, int nt, int cap, int sms, int slots) {
+    std::vector<std::pair<int, int>> sizes;
+    for (const Req *r : sv->active) sizes.push_back({r->p.Lx, r->p.Ly});
+    if (nt < 0) return swb::pair_iteration_us(sizes, nt, cap, sms, slots);
+    const bool f64 = sv->precision == SWB_F64;
+    double cells = 0.0;
     int tallest = 0;
-    for (const Req *r : sv->active) {
-        const int h = balanced_rows(r->p.Ly, cap);
-        const double n = (double)((r->p.Lx + w - 1) / w) * (double)((r->p.Ly + h - 1) / h);
+    for (const auto &p : sizes) {
+        const int h = swb::balanced_rows(p.second, cap), w = nt - 4;
         tallest = std::max(tallest, h);
-        strips += n;
-        cells += n * (w + 4) * (h + 4);
+        cells += (double)((p.first + w - 1) / w) * nt * (double)((p.second + h - 1) / h) * (h + 4);
     }
-    if (nt >= 0) {
-        const bool f64 = sv->precision == SWB_F64;
-        return std::max((tallest + 4) * (f64 ? 10.0 : 0.6), cells / (f64 ? 2e3 : 55e3));
-    }
-    const double c = strips * (-nt / 64.0) / sms;  // CTAs per SM, in units of 64 threads
-    auto row = [](double c) { return 0.655 * (1.0 + 0.17 * std::max(0.0, c - 1.4)); };
-    const double waves = std::floor(c / 8.0), rest = c - 8.0 * waves;
-    return 4.7 + (tallest + 4) * (waves * row(8.0) + (rest > 0.0 ? row(rest) : 0.0));
+    return std::max((tallest + 4) * (f64 ? 10.0 : 0.6), cells / (f64 ? 2e3 : 55e3));
 }
 void choose_geometry(swb_server *sv, int sms) {
     bool pair = sv->precision == SWB_F32 || sv->precision == SWB_F16;
-    for (Req *r : sv->active) pair = pair && r->p.Lx % 2 == 0 && swb::pair_form_ok(r->a);
+    bool wave = false;
+    for (Req *r : sv->active) {
+        pair = pair && r->p.Lx % 2 == 0 && swb::pair_form_ok(r->a);
+        wave = wave || r->a.theta_mode == swb::THETA_WAVE;
+    }
     int best_nt = swb::kBatchNT, best_cap = kServePairRows;
     double best = -1.0;
     for (int nt : {-64, -32, swb::kBatchNT}) {
         if ((nt < 0) != pair || (pair && sv->geo_nt != 0 && nt != sv->geo_nt)) continue;
-        for (int cap : {64, 48, 32, 24, 16, 12, 8, 6, 4, 3, 2}) {
-            if (pair && sv->geo_rows > 0) cap = sv->geo_rows;
-            if (!pair && cap > swb::kBatchRows) continue;
-            const double us = iteration_us(sv, nt, cap, sms);
+        const int slots = pair ? swb::batch_blocks_per_sm(sv->precision, nt, wave) : 0;
+        for (int k = pair ? kServePairRows : swb::kBatchRows; k >= swb::kMinRows; --k) {
+            const int cap = pair && sv->geo_rows > 0 ? sv->geo_rows : k;
+            const double us = iteration_us(sv, nt, cap, sms, slots);
             if (best < 0.0 || us < best) {
                 best = us;
                 best_nt = nt;
@@ -238,7 +226,7 @@ void choose_geometry(swb_server *sv, int sms) {
     }
     sv->nt = best_nt;
     for (Req *r : sv->active)
-        swb::set_geometry(r->a, sv->nt, std::max(balanced_rows(r->p.Ly, best_cap), swb::kMinRows));
+        swb::set_geometry(r->a, sv->nt, std::max(swb::balanced_rows(r->p.Ly, best_cap), swb::kMinRows));
 }
 
 // Packed table of (lattice, strip) entries, the lattices' reducers first.
