@@ -16,6 +16,7 @@ from typing import Callable, Optional, Sequence
 import numpy as np
 
 from . import _lib as L
+from . import _results
 from ._lib import check, lib
 
 _GREEK = {"τ": "tau", "cₛ": "cs", "μ": "mu", "δ": "delta", "γ": "gamma", "θ": "theta"}
@@ -145,7 +146,7 @@ class GB300State:
         column-major, the field's shape; e.g. pinned host memory)."""
         shape = self.shape + ((9,) if name in ("fout", "feq") else ())
         if out is None:
-            out = np.empty(shape, dtype=np.float64, order="F")
+            out = _results.empty(shape)
         elif out.shape != shape or out.dtype != np.float64 or not out.flags.f_contiguous:
             raise ValueError(f"out must be a column-major Float64 array of shape {shape}")
         self._chk(lib().swb_get_field(self._h, L.FIELD[name], out.ctypes.data))
@@ -796,7 +797,7 @@ class Batch:
 
     def get_height(self, i: int) -> np.ndarray:
         s = self.systems[i]
-        out = np.empty((s.Lx, s.Ly), order="F")
+        out = _results.empty((s.Lx, s.Ly))
         check(lib().swb_batch_get_height(self._h, i, out.ctypes.data))
         return out
 
