@@ -11,17 +11,16 @@
 // in the reference's operation order (this unit is compiled with
 // --fmad=false), so Float64 results equal the oracle's bit for bit.
 //
-// A Float64 iteration of 128 cells takes an SM about 2 us (its Float64 units
-// finish a warp instruction every 16 cycles), whatever else is done, so the
-// cells of a lattice are spread over the SMs: a CTA of 128 threads, one cell
-// each, runs K iterations in registers and shared memory on its own cells and
-// a halo of 3 K cells on either side (an iteration reaches 3 cells: pressure,
-// force, streaming), recomputing the halo instead of exchanging it, and writes
-// its own cells to the other set of buffers.  (One CTA for a whole lattice
-// took 26.8 us per Float64 iteration of 1024 cells; this takes 3.3, with the
-// call's upload and reads.)  No CTA waits for another, and a
-// launch is paid once per K iterations.  Lattices of at most 128 cells fit one
-// CTA with no halo.
+// An SM's Float64 units take about 2 us for a Float64 iteration of 128 cells,
+// whatever else is done, so the cells of a lattice are spread over the SMs: a CTA
+// of 64 or 128 cells, one or two threads each, runs K iterations in registers
+// and shared memory on its own cells and a halo of 3 K cells on either side (an
+// iteration reaches 3 cells: pressure, force, streaming), recomputing the halo
+// instead of exchanging it, and writes its own cells to the other set of
+// buffers.  (One CTA for a whole lattice took 26.8 us per Float64 iteration of
+// 1024 cells; this takes 2.0.)  No CTA waits for another, and a launch is paid
+// once per K iterations.  Lattices of at most that many cells fit one CTA with
+// no halo.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -35,7 +34,9 @@
 
 namespace swb {
 
-constexpr int kD1NT = 128;
+// Cells of a CTA, halo included: kD1Cells, or half as many where that spreads a
+// Float64 lattice over more SMs (one warp per SM quarter, see D1Ops64).
+constexpr int kD1Cells = 128;
 
 struct D1Args {
     int L;
@@ -136,18 +137,28 @@ __device__ __noinline__ void d1_second_again(const D1Cell<double> &c, double h, 
 __device__ __noinline__ void d1_moments_again(const double *f, double *h, double *u) {
     D1Cell64<Plain64>{}.moments(f, *h, *u);
 }
+// Products in integers (Fast64), or with FAST = D1Direct64 on the Float64 unit:
+// alone on an SM quarter a warp waits 64 cycles for a Float64 product and 113
+// for one in integers (64 cells per CTA: 1.75 and 2.34 us per iteration; 128
+// cells, two warps per quarter: 2.6 either way).
+struct D1Direct64 : Fast64 {
+    using Fast64::Fast64;
+    __device__ __forceinline__ double mul(double a, double b) const { return a * b; }
+    __device__ __forceinline__ double muln(double a, double b) const { return a * b; }
+};
+template <class FAST>
 struct D1Ops64 {
     Fma64 f;
     __device__ __forceinline__ double pressure(const D1Args &a, const D1Cell<double> &c, double h, double hip,
                                                double him) const {
-        D1Cell64<Fast64> k{Fast64(f)};
+        D1Cell64<FAST> k{FAST(f)};
         const double p = k.pressure(a, c, h, hip, him);
         if (!k.o.bad) return p;
         const D1Cell<double> cc = c;
         return d1_pressure_again(a, cc, h, hip, him);
     }
     __device__ __forceinline__ void local(const D1Cell<double> &c, double h, double u, D1Mid<double> &m) const {
-        D1Cell64<Fast64> k{Fast64(f)};
+        D1Cell64<FAST> k{FAST(f)};
         k.local(c, h, u, m);
         if (k.o.bad) {
             const D1Cell<double> cc = c;
@@ -158,7 +169,7 @@ struct D1Ops64 {
     }
     __device__ __forceinline__ void second(const D1Cell<double> &c, double h, const D1Mid<double> &m, double pm,
                                            double pp, const double fo[3], double out[3]) const {
-        D1Cell64<Fast64> k{Fast64(f)};
+        D1Cell64<FAST> k{FAST(f)};
         k.second(c, h, m, pm, pp, fo, out);
         if (k.o.bad) {
             const D1Cell<double> cc = c;
@@ -171,7 +182,7 @@ struct D1Ops64 {
         }
     }
     __device__ __forceinline__ void moments(const double fo[3], double &h, double &u) const {
-        D1Cell64<Fast64> k{Fast64(f)};
+        D1Cell64<FAST> k{FAST(f)};
         k.moments(fo, h, u);
         if (k.o.bad) {
             const double in[3] = {fo[0], fo[1], fo[2]};
@@ -251,28 +262,28 @@ __device__ __forceinline__ void d1_measure(D1Part *out, bool own, double h, bool
 }
 
 // n iterations of the cells of chunk blockIdx.x, from the buffers `from` to the
-// others.  part: this launch's measures, [n][gridDim.x][kD1NT / 32] (or null).
-// Float64 has two threads per cell: the first kD1NT compute pressures (and the
+// others.  part: this launch's measures, [n][gridDim.x][NT / 32] (or null).
+// Float64 has two threads per cell: the first NT compute pressures (and the
 // measures) while the others compute slippage and equilibrium, the two long
 // chains of an iteration, and then collide and stream (2.82 -> 2.58 us per
 // iteration; FP32, whose chains are short, 0.94 -> 0.97 and so one thread).
 template <class R>
 constexpr int kD1Halves = sizeof(R) == 8 ? 2 : 1;
-template <class R, class Ops>
-__global__ void __launch_bounds__(kD1Halves<R> * kD1NT) d1q3_run_kernel(const D1Args *__restrict__ args,
+template <class R, class Ops, int NT>
+__global__ void __launch_bounds__(kD1Halves<R> * NT) d1q3_run_kernel(const D1Args *__restrict__ args,
                                                          const D1Chunk *__restrict__ table, const Ops op,
                                                          int from, int n, D1Part *part) {
     __shared__ D1Args a;
-    __shared__ R sh[kD1NT], sp[kD1NT], s1[kD1NT], s2[kD1NT];
+    __shared__ R sh[NT], sp[NT], s1[NT], s2[NT];
     const D1Chunk ck = table[blockIdx.x];
     if (threadIdx.x == 0) a = args[ck.lattice];
     __syncthreads();
     grid_dep_wait();
     grid_dep_launch();
-    const int t = threadIdx.x & (kD1NT - 1), L = a.L;
-    const bool first = threadIdx.x < kD1NT;  // computes pressures (whole warps)
+    const int t = threadIdx.x & (NT - 1), L = a.L;
+    const bool first = threadIdx.x < NT;  // computes pressures (whole warps)
     const bool second = kD1Halves<R> == 1 || !first;  // holds the cell's state
-    const bool whole = ck.w == L && L <= kD1NT;  // periodic within the CTA
+    const bool whole = ck.w == L && L <= NT;  // periodic within the CTA
     const int halo = whole ? 0 : 3 * n, span = ck.w + 2 * halo;
     const bool in = t < span, own = t >= halo && t < halo + ck.w;
     int g = ck.x0 - halo + t;  // halo < L
@@ -312,7 +323,7 @@ __global__ void __launch_bounds__(kD1Halves<R> * kD1NT) d1q3_run_kernel(const D1
                 sp[t] = p;
             }
             if (rec)
-                d1_measure(part + ((size_t)k * gridDim.x + blockIdx.x) * (kD1NT / 32) + (t >> 5), own, (double)hc,
+                d1_measure(part + ((size_t)k * gridDim.x + blockIdx.x) * (NT / 32) + (t >> 5), own, (double)hc,
                            hc > R(0.055));
         }
         if (second && in) {
@@ -349,7 +360,7 @@ __global__ void __launch_bounds__(kD1Halves<R> * kD1NT) d1q3_run_kernel(const D1
 // per lattice (blockIdx.y) and iteration.
 __global__ void __launch_bounds__(128) d1q3_record_kernel(const D1Args *__restrict__ args,
                                                           const D1Part *__restrict__ part, int nchunks,
-                                                          int n, long long t0) {
+                                                          int warps, int n, long long t0) {
     const D1Args &a = args[blockIdx.y];
     const int k = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (k >= n || !a.rec || n - k > a.rec_cap) return;  // only the newest the ring holds
@@ -357,8 +368,8 @@ __global__ void __launch_bounds__(128) d1q3_record_kernel(const D1Args *__restri
     unsigned long long mx = 0, mn = 0;
     int wet = 0;
     double big = 0.0;
-    const D1Part *pp = part + ((size_t)k * nchunks + a.chunk0) * (kD1NT / 32);
-    for (int i = lane; i < a.chunks * (kD1NT / 32); i += 32) {
+    const D1Part *pp = part + ((size_t)k * nchunks + a.chunk0) * warps;
+    for (int i = lane; i < a.chunks * warps; i += 32) {
 #pragma unroll
         for (int q = 0; q < kChunks; ++q)
             c[q] += q == kChunks - 1 ? (long long)(int32_t)pp[i].mass[q] : (long long)pp[i].mass[q];
@@ -424,6 +435,7 @@ struct swb1d {
     swb::D1Chunk *d_chunks = nullptr;
     int nchunks = 0;
     int per_launch = 0;        // iterations a launch may run
+    int cells = swb::kD1Cells;  // cells of a CTA, halo included
     swb::D1Part *d_part = nullptr;
     int part_steps = 0;        // iterations d_part holds
     bool args_dirty = true;
@@ -517,33 +529,39 @@ constexpr size_t kPartBytes = (size_t)64 << 20;  // of measures a burst keeps
 
 // Cuts the lattices into chunks of one CTA each and returns the iterations K
 // of a launch.  A launch of c CTAs per SM lasts about K max(1, c / r) t + t0:
-// Float64 t = 2 us and r = 1 (one CTA keeps an SM's Float64 units busy), FP32
-// t = 0.6 us and r = 8 (it leaves them idle), t0 = 2 us; larger K need more
-// CTAs, because 6 K of their 128 cells are halo.
+// Float64 t = 2.5 us with CTAs of 128 cells and 1.75 with 64, r = 1 (one CTA keeps
+// an SM's Float64 units busy), FP32 t = 0.9 us and r = 8 (it leaves them idle),
+// t0 = 2 us; larger K need more CTAs, because 6 K of their cells are halo.
 int split_lattices(swb1d *b, std::vector<swb::D1Chunk> &out) {
     int sms = 1, dev = 0;
     cudaGetDevice(&dev);
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 1;
-    const double t = b->rb == 8 ? 2.0 : 0.6, r = b->rb == 8 ? 1.0 : 8.0;
-    auto pieces = [&](int L, int K) {
-        const int w = swb::kD1NT - 6 * K;
-        return L <= swb::kD1NT ? 1 : (L + w - 1) / w;
+    const bool f64 = b->rb == 8;
+    auto pieces = [](int L, int cells, int K) {
+        const int w = cells - 6 * K;
+        return L <= cells ? 1 : (L + w - 1) / w;
     };
-    int best = 1;
+    int best = 1, cells = swb::kD1Cells;
     double cost = 1e300;
-    bool small = true;
-    for (const swb_params &p : b->params) small = small && p.Lx <= swb::kD1NT;
-    for (int K = 1; K <= 19; ++K) {
-        long long n = 0;
-        for (const swb_params &p : b->params) n += pieces(p.Lx, K);
-        const double c = std::max(1.0, std::ceil((double)n / sms) / r) * t + 2.0 / K;
-        if (c < cost) {
-            cost = c;
-            best = K;
+    for (int nt : {swb::kD1Cells, swb::kD1Cells / 2}) {
+        if (nt != swb::kD1Cells && !f64) break;
+        const double t = !f64 ? 0.9 : (nt == swb::kD1Cells ? 2.5 : 1.75), r = f64 ? 1.0 : 8.0;
+        for (int K = 1; 6 * K + 8 <= nt; ++K) {
+            long long n = 0;
+            for (const swb_params &p : b->params) n += pieces(p.Lx, nt, K);
+            const double c = std::max(1.0, std::ceil((double)n / sms) / r) * t + 2.0 / K;
+            if (c < cost) {
+                cost = c;
+                best = K;
+                cells = nt;
+            }
         }
     }
+    b->cells = cells;
+    bool small = true;
+    for (const swb_params &p : b->params) small = small && p.Lx <= cells;
     for (int i = 0; i < b->count; ++i) {
-        const int L = b->params[i].Lx, k = pieces(L, best);
+        const int L = b->params[i].Lx, k = pieces(L, cells, best);
         b->args[i].chunk0 = (int)out.size();
         b->args[i].chunks = k;
         for (int j = 0; j < k; ++j) {
@@ -718,7 +736,8 @@ int swb1d_step(swb1d *b, int64_t nsteps) {
         b->args_dirty = false;
     }
     // bursts of launches, then the burst's records
-    const size_t row = sizeof(swb::D1Part) * (swb::kD1NT / 32) * (size_t)b->nchunks;
+    const int warps = b->cells / 32;
+    const size_t row = sizeof(swb::D1Part) * warps * (size_t)b->nchunks;
     while (nsteps > 0) {
         int burst = (int)std::min<int64_t>(nsteps, kBurst);
         if (b->rec_cap) {
@@ -735,15 +754,19 @@ int swb1d_step(swb1d *b, int64_t nsteps) {
         for (int done = 0; done < burst;) {
             const int n = std::min(b->per_launch, burst - done);
             swb::D1Part *part =
-                b->rec_cap ? b->d_part + (size_t)done * b->nchunks * (swb::kD1NT / 32) : nullptr;
+                b->rec_cap ? b->d_part + (size_t)done * b->nchunks * warps : nullptr;
             const swb::Fma64 f{1.0};
             auto run = [&](auto *kern, int halves, auto ops) {
-                return swb::launch_step(kern, b->nchunks, halves * swb::kD1NT, b->stream, b->d_args, b->d_chunks, ops,
+                return swb::launch_step(kern, b->nchunks, halves * b->cells, b->stream, b->d_args, b->d_chunks, ops,
                                         b->cur, n, part);
             };
+            using Split = swb::D1Ops64<swb::Fast64>;
+            using Direct = swb::D1Ops64<swb::D1Direct64>;
+            constexpr int C = swb::kD1Cells;
             const cudaError_t e =
-                b->rb == 8 ? run(swb::d1q3_run_kernel<double, swb::D1Ops64>, swb::kD1Halves<double>, swb::D1Ops64{f})
-                           : run(swb::d1q3_run_kernel<float, swb::D1Ops32>, swb::kD1Halves<float>, swb::D1Ops32{f});
+                b->rb == 4       ? run(swb::d1q3_run_kernel<float, swb::D1Ops32, C>, swb::kD1Halves<float>, swb::D1Ops32{f})
+                : b->cells == C ? run(swb::d1q3_run_kernel<double, Split, C>, swb::kD1Halves<double>, Split{f})
+                                : run(swb::d1q3_run_kernel<double, Direct, C / 2>, swb::kD1Halves<double>, Direct{f});
             D1_TRY(b, e);
             swb::count_launches(1);
             b->cur ^= 1;
@@ -751,7 +774,7 @@ int swb1d_step(swb1d *b, int64_t nsteps) {
         }
         if (b->rec_cap) {
             swb::d1q3_record_kernel<<<dim3((unsigned)((burst + 3) / 4), (unsigned)b->count), 128, 0, b->stream>>>(
-                b->d_args, b->d_part, b->nchunks, burst, b->t);
+                b->d_args, b->d_part, b->nchunks, warps, burst, b->t);
             swb::count_launches(1);
             D1_TRY(b, cudaGetLastError());
         }
