@@ -45,16 +45,28 @@ struct LdCG {
     __device__ __forceinline__ static T ld(const T *p) { return __ldcg(p); }
 };
 
+// Element i of a plane of T: the plane's address is the same for every thread,
+// so with an unsigned 32-bit byte offset (9 planes stay below 2^31 elements)
+// an access needs no 64-bit address arithmetic of its own.
+template <class T>
+__device__ __forceinline__ const T *at(const T *plane, int i) {
+    return reinterpret_cast<const T *>(reinterpret_cast<const char *>(plane) + (unsigned)i * (unsigned)sizeof(T));
+}
+template <class T>
+__device__ __forceinline__ T *at(T *plane, int i) {
+    return reinterpret_cast<T *>(reinterpret_cast<char *>(plane) + (unsigned)i * (unsigned)sizeof(T));
+}
+
 template <class L>
 struct StoreF64T {
     using real = double;
     static constexpr bool kLiteral = true;
     static constexpr bool kHalf = false;
     __device__ __forceinline__ static double ld(const void *b, int pitch, int q, int i) {
-        return L::ld(reinterpret_cast<const double *>(b) + q * pitch + i);
+        return L::ld(at(reinterpret_cast<const double *>(b) + q * pitch, i));
     }
     __device__ __forceinline__ static void st(void *b, int pitch, int q, int i, double v) {
-        reinterpret_cast<double *>(b)[q * pitch + i] = v;
+        *at(reinterpret_cast<double *>(b) + q * pitch, i) = v;
     }
 };
 
@@ -64,10 +76,10 @@ struct StoreF32T {
     static constexpr bool kLiteral = false;
     static constexpr bool kHalf = false;
     __device__ __forceinline__ static float ld(const void *b, int pitch, int q, int i) {
-        return L::ld(reinterpret_cast<const float *>(b) + q * pitch + i);
+        return L::ld(at(reinterpret_cast<const float *>(b) + q * pitch, i));
     }
     __device__ __forceinline__ static void st(void *b, int pitch, int q, int i, float v) {
-        reinterpret_cast<float *>(b)[q * pitch + i] = v;
+        *at(reinterpret_cast<float *>(b) + q * pitch, i) = v;
     }
 };
 
@@ -84,15 +96,15 @@ struct StoreF16T {
         return reinterpret_cast<const __half *>(reinterpret_cast<const float *>(b) + pitch);
     }
     __device__ __forceinline__ static float ld(const void *b, int pitch, int q, int i) {
-        if (q == 0) return L::ld(reinterpret_cast<const float *>(b) + i);
-        return __half2float(L::ld(hp(b, pitch) + (q - 1) * pitch + i)) * kInv;
+        if (q == 0) return L::ld(at(reinterpret_cast<const float *>(b), i));
+        return __half2float(L::ld(at(hp(b, pitch) + (q - 1) * pitch, i))) * kInv;
     }
     __device__ __forceinline__ static void st(void *b, int pitch, int q, int i, float v) {
         if (q == 0) {
-            reinterpret_cast<float *>(b)[i] = v;
+            *at(reinterpret_cast<float *>(b), i) = v;
         } else {
             __half *h = const_cast<__half *>(hp(b, pitch));
-            h[(q - 1) * pitch + i] = __float2half_rn(v * kScale);
+            *at(h + (q - 1) * pitch, i) = __float2half_rn(v * kScale);
         }
     }
 };
@@ -479,11 +491,12 @@ __device__ __forceinline__ void mass_add(PartQ &p, float v) {
     p.mq += __float2ll_rn(v * kMassScale);
 }
 
-// The rounding residue of a cell's pulled height (a few ulp of h).
+// The rounding residue of a cell's pulled height (a few ulp of h, far below the
+// 0.5 that 32 bits hold; the 32-bit conversion is the faster one).
 template <class R>
 __device__ __forceinline__ void mass_add_lo(PartT<R> &p, R lo) { p.mlo = p.mlo + lo; }
 __device__ __forceinline__ void mass_add_lo(PartQ &p, float lo) {
-    p.mq += __float2ll_rn(lo * kMassScale);
+    p.mq += __float2int_rn(lo * kMassScale);
 }
 
 // A wetted cell's surface element and cos θ (surfacearea!, src/measures.jl).
@@ -1117,12 +1130,12 @@ __device__ __forceinline__ void collide_cell(const StepArgs &a,
         collide_fast<S, FRESH, TAU1, true>(cc, h, ux, uy, Fx, Fy, hft, fq, cell, tt, hlo_p, fo, hb);
         if constexpr (S::kHalf) {
             reinterpret_cast<float *>(dst)[cell] = fo[0];
-            __half *hpl = const_cast<__half *>(S::hp(dst, pitch)) + cell;
+            __half *hpl = const_cast<__half *>(S::hp(dst, pitch));
             // planes 1..8 in the order of hb: (1, 2), (3, 4), (5, 6), (7, 8)
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                hpl[(2 * k) * pitch] = __low2half(hb[k]);
-                hpl[(2 * k + 1) * pitch] = __high2half(hb[k]);
+                *at(hpl + (2 * k) * pitch, cell) = __low2half(hb[k]);
+                *at(hpl + (2 * k + 1) * pitch, cell) = __high2half(hb[k]);
             }
         } else {
 #pragma unroll
@@ -1373,24 +1386,24 @@ struct PairPull {
 
 template <class S>
 __device__ __forceinline__ float2 pair_f0(const void *b, int i) {
-    return __ldg(reinterpret_cast<const float2 *>(reinterpret_cast<const float *>(b) + i));
+    return __ldg(reinterpret_cast<const float2 *>(at(reinterpret_cast<const float *>(b), i)));
 }
 
 // plane q (1..8) at element i (even): the pair as stored
 template <class S>
 __device__ __forceinline__ typename PairPull<S>::W pair_ld(const void *b, int pitch, int q, int i) {
     if constexpr (S::kHalf)
-        return __ldg(reinterpret_cast<const __half2 *>(S::hp(b, pitch) + (q - 1) * pitch + i));
+        return __ldg(reinterpret_cast<const __half2 *>(at(S::hp(b, pitch) + (q - 1) * pitch, i)));
     else
-        return __ldg(reinterpret_cast<const float2 *>(reinterpret_cast<const float *>(b) + q * pitch + i));
+        return __ldg(reinterpret_cast<const float2 *>(at(reinterpret_cast<const float *>(b) + q * pitch, i)));
 }
 
 template <class S>
 __device__ __forceinline__ typename PairPull<S>::E one_ld(const void *b, int pitch, int q, int i) {
     if constexpr (S::kHalf)
-        return __ldg(S::hp(b, pitch) + (q - 1) * pitch + i);
+        return __ldg(at(S::hp(b, pitch) + (q - 1) * pitch, i));
     else
-        return __ldg(reinterpret_cast<const float *>(b) + q * pitch + i);
+        return __ldg(at(reinterpret_cast<const float *>(b) + q * pitch, i));
 }
 
 // The pulled values of a plane at the pair, (f_q(c), f_q(c + 1)), from the
@@ -1422,8 +1435,8 @@ __device__ __forceinline__ __half shfl_lo_down(__half2 w) {
 
 // One iteration on pair strip (bx, by): thread t owns columns c = x0 - 2 + 2t
 // and c + 1 and marches the strip's rows with shared-memory rings of pairs,
-// as march_run does with one column.  Strips of odd index march up, the
-// others down (below).  Measured on GB300 (A/B on one box): the 512-member
+// as march_run does with one column.  Strips of odd index march one way, the
+// others the other (below).  Measured on GB300 (A/B on one box): the 512-member
 // ensemble 74.8k -> 78.0k MLUPS; a single 2048² lattice (one wave of strips)
 // FP32 53.3 us either way, FP16 storage 55.7 -> 54.7 us.  Results are the
 // same bits (the per-cell arithmetic and each cell's neighbours do not
@@ -1449,7 +1462,7 @@ __device__ __forceinline__ void march2_run(const StepArgs &a, int bx, int by, lo
     auto wrow = [&](int yy) {
         return tiny_y ? wrapc(yy, Ly) : (yy < 0 ? yy + Ly : (yy >= Ly ? yy - Ly : yy));
     };
-    // Strips of odd index march up, the others down, so that two strips
+    // Strips of odd index march one way, the others the other, so that two strips
     // adjacent in y pull the rows they share (each strip's 2 halo rows on
     // either side) at about the same time, while L2 still holds them,
     // instead of one at the start and the other at the end of its march.
@@ -1457,7 +1470,10 @@ __device__ __forceinline__ void march2_run(const StepArgs &a, int bx, int by, lo
     // rows -2, -1, rows, rows + 1); ring(yy): its ring slot, m + 2 either
     // way.  In the rings the previous march row is the row above (y - 1)
     // when marching down and the row below (y + 1) when marching up.
-    const bool up = (by & 1) != 0;
+    // The directions change with every iteration, so that a march begins with
+    // the rows the previous iteration wrote last, which L2 still holds (2048²
+    // FP32 54.9 -> 54.2 us, FP16 storage 54.2 -> 53.4).
+    const bool up = ((by ^ (int)done) & 1) != 0;
     auto Y = [&](int m) { return up ? y0 + rows - 1 - m : y0 + m; };
     auto ring = [&](int yy) { return up ? y0 + rows + 1 - yy : yy - y0 + 2; };
     // this thread's pair (c, c + 1); x0 and Lx are even
@@ -1483,10 +1499,36 @@ __device__ __forceinline__ void march2_run(const StepArgs &a, int bx, int by, lo
     const int tl = t > 0 ? 2 * t - 1 : 0, tr = t < NT - 1 ? 2 * t + 2 : 2 * NT - 1;
 
     PP fa_, fb_;
-    auto issue = [&](PP &P, int yy) {
-        const int gy = wrow(yy);
-        const int gym = gy == 0 ? Ly - 1 : gy - 1, gyp = gy == Ly - 1 ? 0 : gy + 1;
-        const int rc = gy * Lx, rm = gym * Lx, rp = gyp * Lx;
+    // FP16 planes: offsets of the rows above, at and below the next row to pull,
+    // moved on a row at a time (2048² 51.8 -> 50.3 us).  FP32 has no registers to
+    // spare for them and computes each row's.
+    int oM = 0, oC = 0, oP = 0;
+    const int lastrow = (Ly - 1) * Lx;
+    if constexpr (S::kHalf) {
+        const int gy = wrapc(Y(-2), Ly);
+        oC = gy * Lx;
+        oM = (gy == 0 ? Ly - 1 : gy - 1) * Lx;
+        oP = (gy == Ly - 1 ? 0 : gy + 1) * Lx;
+    }
+    auto issue = [&](PP &P, int yy) {  // rows are issued in march order
+        int rc = oC, rm = oM, rp = oP;
+        if constexpr (S::kHalf) {
+            if (up) {
+                oP = oC;
+                oC = oM;
+                oM = oM == 0 ? lastrow : oM - Lx;
+            } else {
+                oM = oC;
+                oC = oP;
+                oP = oP == lastrow ? 0 : oP + Lx;
+            }
+        } else {
+            const int gy = wrow(yy);
+            const int gym = gy == 0 ? Ly - 1 : gy - 1, gyp = gy == Ly - 1 ? 0 : gy + 1;
+            rc = gy * Lx;
+            rm = gym * Lx;
+            rp = gyp * Lx;
+        }
         P.f0 = pair_f0<S>(src, rc + cx);
         P.q[0] = pair_ld<S>(src, pitch, 1, rc + cx);  // f1 from x - 1
         P.q[1] = pair_ld<S>(src, pitch, 2, rm + cx);  // f2 from y - 1
@@ -1591,7 +1633,7 @@ __device__ __forceinline__ void march2_run(const StepArgs &a, int bx, int by, lo
         if (!interior) continue;
         // ---- output row y, columns cx, cx + 1 ----
         const int r = ring(y);
-        const int cellA = wrow(y) * Lx + cx;
+        const int cellA = (S::kHalf ? y : wrow(y)) * Lx + cx;
         const float2 h2 = sm.h[r & 7][t], jx2 = sm.jx[r & 3][t], jy2 = sm.jy[r & 3][t];
         const float2 lo2 = sm.lo[r & 3][t];
         const float2 *pm = sm.p[(r + 3) & 3], *pc = sm.p[r & 3], *pp = sm.p[(r + 1) & 3];
@@ -1621,20 +1663,18 @@ __device__ __forceinline__ void march2_run(const StepArgs &a, int bx, int by, lo
             collide_fast<S, false, true, true>(cc, h2.y, ux, uy, F.x, F.y, h2.y, nullptr, cellA + 1, tt,
                                          &lo2.y, foB, hbB);
         }
-        reinterpret_cast<float2 *>(reinterpret_cast<float *>(dst) + cellA)[0] = f2(foA[0], foB[0]);
+        *reinterpret_cast<float2 *>(at(reinterpret_cast<float *>(dst), cellA)) = f2(foA[0], foB[0]);
         if constexpr (S::kHalf) {
-            __half2 *hpl = reinterpret_cast<__half2 *>(const_cast<__half *>(S::hp(dst, pitch)) + cellA);
-            const int pitch2 = pitch >> 1;  // pitch in pairs (pitch is a multiple of 64)
+            __half *hpl = const_cast<__half *>(S::hp(dst, pitch));
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                hpl[(2 * k) * pitch2] = __lows2half2(hbA[k], hbB[k]);
-                hpl[(2 * k + 1) * pitch2] = __highs2half2(hbA[k], hbB[k]);
+                *reinterpret_cast<__half2 *>(at(hpl + (2 * k) * pitch, cellA)) = __lows2half2(hbA[k], hbB[k]);
+                *reinterpret_cast<__half2 *>(at(hpl + (2 * k + 1) * pitch, cellA)) = __highs2half2(hbA[k], hbB[k]);
             }
         } else {
-            float2 *d2 = reinterpret_cast<float2 *>(reinterpret_cast<float *>(dst) + cellA);
-            const int pitch2 = pitch >> 1;
 #pragma unroll
-            for (int q = 1; q < 9; ++q) d2[q * pitch2] = f2(foA[q], foB[q]);
+            for (int q = 1; q < 9; ++q)
+                *reinterpret_cast<float2 *>(at(reinterpret_cast<float *>(dst) + q * pitch, cellA)) = f2(foA[q], foB[q]);
         }
         // measures of the heights at the start of this iteration
         if (!isfinite(h2.x) || !isfinite(h2.y)) any_nan = 1;
