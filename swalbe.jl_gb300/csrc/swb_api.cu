@@ -658,8 +658,8 @@ cudaError_t launch_sequence(swb_state *s, int n) {
 // Autotuner: times a few geometries and launch forms on real steps (each
 // probe is a complete launch sequence, so nothing is wasted) and keeps the
 // fastest.  Every candidate first runs a short untimed sequence, which also
-// loads its kernel (modules load lazily, on first launch).  Only for
-// SWB_F64 / SWB_F32, whose results do not depend on the geometry.
+// loads its kernel (modules load lazily, on first launch).  SWB_F32 and
+// SWB_F16, whose results do not depend on the geometry; SWB_F64 has none.
 constexpr int kTuneMinSteps = 512;
 constexpr int kTuneProbe = 16;
 constexpr int kPersistProbe = 4;

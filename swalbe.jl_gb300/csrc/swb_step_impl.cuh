@@ -1376,8 +1376,8 @@ struct PairSmem {
 // Blackwell's packed FP32 operations.  Each lane goes through the operations of
 // moments9 and moments_lo in their order (a - b as fma(-1, b, a)), so the bits
 // are theirs; the pairs are the columns' own, as loaded and as stored, so no
-// instruction is spent on forming them.  2048² FP32 53.1 -> 52.9 us, FP16
-// storage 49.8 -> 48.3.  The pressure and the collision stay scalar: packed as
+// instruction is spent on forming them.  2048² FP32 53.3 -> 53.1 us, FP16
+// storage 50.4 -> 49.0.  The pressure and the collision stay scalar: packed as
 // well they gave FP16 47.7 us, but FP32 strips of 64 threads 56.2.
 __device__ __forceinline__ float2 small8_2(const float2 f[9]) {
     return add2(add2(add2(f[1], f[3]), add2(f[5], f[7])), add2(add2(f[2], f[4]), add2(f[6], f[8])));
