@@ -2,7 +2,8 @@
 // a*b+c is contracted into an FMA: the reference (Julia broadcasts) rounds
 // every operation, and this translation unit reproduces it bit for bit.
 //
-// Contents: the fused step in Float64 (literal arithmetic), the plain
+// Contents: the cell kernels of single lattices, the strips of batched and
+// served ones (literal arithmetic), θ fields, the plain
 // one-kernel-per-reference-op path, and the standalone measure reduction.
 #include "swb_step_impl.cuh"
 #include "swb_f64.cuh"
@@ -785,6 +786,15 @@ __global__ void k_bgk_stream(PlainState s, Fma64 g, double omeg, double invtau) 
     }
 }
 
+__global__ void k_copy_streamed(PlainState s) {
+    grid_dep_wait();
+    grid_dep_launch();
+    PLAIN_LOOP(s) {
+#pragma unroll
+        for (int q = 0; q < 9; ++q) s.fout[q * s.N + c] = s.ftemp[q * s.N + c];
+    }
+}
+
 __global__ void k_moments(PlainState s, Fma64 g) {
     grid_dep_wait();
     grid_dep_launch();
@@ -846,13 +856,19 @@ cudaError_t plain_equilibrium(const PlainState &s, double g, cudaStream_t st) {
 }
 cudaError_t plain_bgk_stream(PlainState &s, double omeg, double invtau, cudaStream_t st) {
     count_launches(1);
-    const cudaError_t e = launch_step(k_bgk_stream, grid_for(s.N, kPlainNT), kPlainNT, st, s,
-                                      Fma64{1.0}, omeg, invtau);
-    if (e == cudaSuccess) {
-        double *f = s.fout;
-        s.fout = s.ftemp;
-        s.ftemp = f;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cudaError_t e = launch_step(k_bgk_stream, grid_for(s.N, kPlainNT), kPlainNT, st, s, Fma64{1.0}, omeg, invtau);
+    if (e == cudaSuccess) e = cudaStreamIsCapturing(st, &cap);
+    if (e != cudaSuccess) return e;
+    if (cap == cudaStreamCaptureStatusActive) {
+        // a caller's graph is replayed with the buffers of its capture, any
+        // number of times: the result goes back to where it was read
+        count_launches(1);
+        return launch_step(k_copy_streamed, grid_for(s.N, kPlainNT), kPlainNT, st, s);
     }
+    double *f = s.fout;
+    s.fout = s.ftemp;
+    s.ftemp = f;
     return e;
 }
 cudaError_t plain_moments(const PlainState &s, cudaStream_t st) { PLAIN_LAUNCH(k_moments, s, st); }
