@@ -40,7 +40,17 @@ def _take(size: int):
             if len(_free[i]) == size:
                 _kept -= size
                 return _free.pop(i)
-    return mmap.mmap(-1, size)
+    # private, as numpy's own memory is: after a fork each process writes to its
+    # own copy (and, as for numpy's, in large pages where the system has them)
+    try:
+        mem = mmap.mmap(-1, size, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
+    except OSError as e:
+        raise MemoryError(f"{size} bytes for a result: {e}") from e
+    try:
+        mem.madvise(mmap.MADV_HUGEPAGE)
+    except (AttributeError, OSError):
+        pass
+    return mem
 
 
 def empty(shape) -> np.ndarray:
