@@ -10,7 +10,9 @@ memory itself (24 results of 0.1 to 2 MiB: 11.9 ms, and 12.2 from here).
 """
 from __future__ import annotations
 
+import collections
 import mmap
+import os
 import threading
 import weakref
 
@@ -19,27 +21,52 @@ import numpy as np
 MIN_BYTES = 32 << 20    # smaller arrays come from numpy's allocator
 KEEP_BYTES = 256 << 20  # unused memory kept at most
 
-_lock = threading.Lock()
+_lock = threading.Lock()  # for _free and _kept; only release() waits for it
+_returned: collections.deque = collections.deque()  # given back, not sorted in yet
 _free: list = []  # unused mappings, oldest first
 _kept = 0
 
 
-def _give(mem) -> None:
+def _sort_in() -> None:
+    """Moves what was given back to the unused mappings, as many as are kept.
+
+    A finalizer runs wherever the garbage collector does, also on a thread that
+    holds the lock, so nothing here waits for it: whoever holds it comes back
+    for what was given back meanwhile.
+    """
     global _kept
-    with _lock:
-        _free.append(mem)
-        _kept += len(mem)
-        while _kept > KEEP_BYTES:
-            _kept -= len(_free.pop(0))  # unmapped with its last reference
+    while _returned and _lock.acquire(blocking=False):
+        try:
+            while _returned:
+                mem = _returned.popleft()
+                _free.append(mem)
+                _kept += len(mem)
+            while _kept > KEEP_BYTES:
+                _kept -= len(_free.pop(0))  # unmapped with its last reference
+        finally:
+            _lock.release()
+
+
+def _give(mem) -> None:
+    _returned.append(mem)
+    _sort_in()
 
 
 def _take(size: int):
     global _kept
-    with _lock:
-        for i in range(len(_free) - 1, -1, -1):
-            if len(_free[i]) == size:
-                _kept -= size
-                return _free.pop(i)
+    mem = None
+    if _lock.acquire(blocking=False):  # else new memory
+        try:
+            for i in range(len(_free) - 1, -1, -1):
+                if len(_free[i]) == size:
+                    mem = _free.pop(i)
+                    _kept -= size
+                    break
+        finally:
+            _lock.release()
+        _sort_in()
+    if mem is not None:
+        return mem
     # private, as numpy's own memory is: after a fork each process writes to its
     # own copy (and, as for numpy's, in large pages where the system has them)
     try:
@@ -68,5 +95,19 @@ def release() -> None:
     """Gives unused memory back."""
     global _kept
     with _lock:
+        _returned.clear()
         _free.clear()
         _kept = 0
+    _sort_in()
+
+
+def _after_fork() -> None:
+    # another thread of the parent may have been inside the pool; it is not here
+    global _lock, _kept
+    _lock = threading.Lock()
+    _returned.clear()
+    _free.clear()
+    _kept = 0
+
+
+os.register_at_fork(after_in_child=_after_fork)

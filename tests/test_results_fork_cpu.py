@@ -47,10 +47,69 @@ print("parent", parent_ok, "child", status)
 
 
 def run(script):
-    r = subprocess.run([sys.executable, "-c", script], cwd=ROOT, capture_output=True, text=True, timeout=120)
+    r = subprocess.run([sys.executable, "-c", script], cwd=ROOT, capture_output=True, text=True, timeout=40)
     assert r.returncode == 0, r.stderr
     return r.stdout.split()
 
 
 def test_a_forked_child_has_its_own_memory():
     assert run(FORK) == ["parent", "True", "child", "0"]
+
+
+CYCLES = """
+import gc, sys, threading
+sys.path.insert(0, "swalbe.jl_gb300")
+from swalbe_gb300 import _results as R
+
+R.release()
+sys.setswitchinterval(1e-5)
+gc.set_threshold(1)
+sizes = [(2048, 2048 + i) for i in range(7)]  # up to seven unused mappings to look through
+
+
+def work():
+    for i in range(2000):
+        cycle = [R.empty(sizes[i % 7])]
+        cycle.append(cycle)  # dropped by the collector, wherever that runs
+        a = R.empty(sizes[(i + 3) % 7])
+        del cycle, a
+
+
+ts = [threading.Thread(target=work) for _ in range(3)]
+for t in ts:
+    t.start()
+for t in ts:
+    t.join()
+gc.set_threshold(700)
+gc.collect()
+R.release()
+print("done", R._kept, len(R._free))
+"""
+
+
+def test_collector_inside_the_pool():
+    """Arrays in reference cycles are given back by the garbage collector, also
+    while this thread takes or gives back other memory."""
+    assert run(CYCLES) == ["done", "0", "0"]
+
+
+HELD = """
+import os, signal, sys
+sys.path.insert(0, "swalbe.jl_gb300")
+from swalbe_gb300 import _results as R
+
+R._lock.acquire()  # another thread is inside the pool when the process forks
+pid = os.fork()
+if pid == 0:
+    signal.alarm(20)
+    a = R.empty((2048, 2048))
+    at = a.ctypes.data
+    del a
+    b = R.empty((2048, 2048))
+    os._exit(0 if b.ctypes.data == at else 3)
+print("child", os.waitstatus_to_exitcode(os.waitpid(pid, 0)[1]))
+"""
+
+
+def test_fork_while_another_thread_is_inside_the_pool():
+    assert run(HELD) == ["child", "0"]
