@@ -306,6 +306,7 @@ struct swb_state {
     StepArgs a{};
     swb::Cell64 x{};  // SWB_F64: the cell kernels' own buffers and constants
     PlainState ps{};
+    bool plain_captured = false;  // an op that uses ps.fout was captured
     double *plain_kapF = nullptr;
     double *plain_cosF = nullptr;  // cospi(θ) of a θ field (the plain path's measures)
     // measures
@@ -525,8 +526,8 @@ int plain_iteration(swb_state *s) {
         CUDA_TRY(&s->err, swb::plain_inclination(ps, s->ax, s->ay, fac, s->stream));
     }
     CUDA_TRY(&s->err, swb::plain_equilibrium(ps, p.g, s->stream));
-    CUDA_TRY(&s->err, swb::plain_bgk_stream(ps, 1.0 - 1.0 / p.tau, 1.0 / p.tau, s->stream));
-    CUDA_TRY(&s->err, swb::plain_moments(ps, s->stream));
+    CUDA_TRY(&s->err, swb::plain_bgk_stream(ps, s->plain_captured, 1.0 - 1.0 / p.tau, 1.0 / p.tau, s->stream));
+    CUDA_TRY(&s->err, swb::plain_moments(ps, s->plain_captured, s->stream));
     s->steps++;
     return SWB_OK;
 }
@@ -1663,12 +1664,13 @@ int swb_op_equilibrium(swb_state *s) {
 }
 int swb_op_bgk_stream(swb_state *s) {
     PLAIN_ONLY(s);
-    CUDA_TRY(&s->err, swb::plain_bgk_stream(s->ps, 1.0 - 1.0 / s->p.tau, 1.0 / s->p.tau, s->stream));
+    CUDA_TRY(&s->err, swb::plain_bgk_stream(s->ps, s->plain_captured, 1.0 - 1.0 / s->p.tau, 1.0 / s->p.tau,
+                                            s->stream));
     return SWB_OK;
 }
 int swb_op_moments(swb_state *s) {
     PLAIN_ONLY(s);
-    CUDA_TRY(&s->err, swb::plain_moments(s->ps, s->stream));
+    CUDA_TRY(&s->err, swb::plain_moments(s->ps, s->plain_captured, s->stream));
     return SWB_OK;
 }
 

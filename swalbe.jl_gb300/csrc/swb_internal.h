@@ -354,8 +354,10 @@ cudaError_t plain_thermal(const PlainState &s, double k6, double delta, unsigned
 cudaError_t plain_inclination(const PlainState &s, double ax, double ay, double fac,
                               cudaStream_t st);
 cudaError_t plain_equilibrium(const PlainState &s, double g, cudaStream_t st);
-cudaError_t plain_bgk_stream(PlainState &s, double omeg, double invtau, cudaStream_t st);  // exchanges fout and ftemp
-cudaError_t plain_moments(const PlainState &s, cudaStream_t st);
+// captured: a caller's graph holds the address of fout, which stays where it is
+// from then on (plain_bgk_stream exchanges fout and ftemp before that)
+cudaError_t plain_bgk_stream(PlainState &s, bool &captured, double omeg, double invtau, cudaStream_t st);
+cudaError_t plain_moments(const PlainState &s, bool &captured, cudaStream_t st);
 
 // Measures of a Float64/float height field: block partials + last-block
 // reduction into `rec` (device).  `scratch` holds blocks*kNPart doubles,

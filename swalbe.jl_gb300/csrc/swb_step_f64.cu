@@ -755,7 +755,7 @@ __global__ void k_equilibrium(PlainState s, Fma64 g, double g56, double g15) {
 // BGKandStream! in one pass: the collision of every cell, each population
 // stored where it streams to (circshift!(ft_q, fo_q, c_q)).  The reference's
 // ftemp equals its fout between ops, so the other buffer takes the result
-// and the caller exchanges the two.
+// and the two are exchanged, or (after a capture) the result is copied back.
 __global__ void k_bgk_stream(PlainState s, Fma64 g, double omeg, double invtau) {
     const int CX[9] = {0, 1, 0, -1, 0, 1, -1, -1, 1};
     const int CY[9] = {0, 0, 1, 0, -1, 1, 1, -1, -1};
@@ -854,15 +854,23 @@ cudaError_t plain_equilibrium(const PlainState &s, double g, cudaStream_t st) {
     auto *const kern = g == 0.0 ? k_equilibrium<true> : k_equilibrium<false>;
     PLAIN_LAUNCH(kern, s, st, (5.0 / 6.0) * g, 1.5 * g);
 }
-cudaError_t plain_bgk_stream(PlainState &s, double omeg, double invtau, cudaStream_t st) {
-    count_launches(1);
+// A captured op that uses fout is replayed with the address of its capture, any
+// number of times and with calls outside the graph in between, so from the first
+// such op on fout is not exchanged any more.
+static cudaError_t note_capture(bool &captured, cudaStream_t st) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    cudaError_t e = launch_step(k_bgk_stream, grid_for(s.N, kPlainNT), kPlainNT, st, s, Fma64{1.0}, omeg, invtau);
-    if (e == cudaSuccess) e = cudaStreamIsCapturing(st, &cap);
+    if (captured) return cudaSuccess;
+    const cudaError_t e = cudaStreamIsCapturing(st, &cap);
+    captured = e == cudaSuccess && cap != cudaStreamCaptureStatusNone;
+    return e;
+}
+cudaError_t plain_bgk_stream(PlainState &s, bool &captured, double omeg, double invtau, cudaStream_t st) {
+    cudaError_t e = note_capture(captured, st);
     if (e != cudaSuccess) return e;
-    if (cap == cudaStreamCaptureStatusActive) {
-        // a caller's graph is replayed with the buffers of its capture, any
-        // number of times: the result goes back to where it was read
+    count_launches(1);
+    e = launch_step(k_bgk_stream, grid_for(s.N, kPlainNT), kPlainNT, st, s, Fma64{1.0}, omeg, invtau);
+    if (e != cudaSuccess) return e;
+    if (captured) {  // the result goes back to where it was read
         count_launches(1);
         return launch_step(k_copy_streamed, grid_for(s.N, kPlainNT), kPlainNT, st, s);
     }
@@ -871,7 +879,11 @@ cudaError_t plain_bgk_stream(PlainState &s, double omeg, double invtau, cudaStre
     s.ftemp = f;
     return e;
 }
-cudaError_t plain_moments(const PlainState &s, cudaStream_t st) { PLAIN_LAUNCH(k_moments, s, st); }
+cudaError_t plain_moments(const PlainState &s, bool &captured, cudaStream_t st) {
+    const cudaError_t e = note_capture(captured, st);
+    if (e != cudaSuccess) return e;
+    PLAIN_LAUNCH(k_moments, s, st);
+}
 
 // ------------------------------------------------------------ measures
 // Grid-stride partials per block, then the last block (ticket) reduces the
