@@ -492,12 +492,12 @@ __device__ __forceinline__ void mass_add(PartQ &p, float v) {
     p.mq += __float2ll_rn(v * kMassScale);
 }
 
-// The rounding residue of a cell's pulled height (a few ulp of h, far below the
-// 0.5 that 32 bits hold; the 32-bit conversion is the faster one).
+// The rounding residue of a cell's pulled height (up to half an ulp of h: 0.5 and
+// more, which 32 bits would not hold, from heights of 2^23 on).
 template <class R>
 __device__ __forceinline__ void mass_add_lo(PartT<R> &p, R lo) { p.mlo = p.mlo + lo; }
 __device__ __forceinline__ void mass_add_lo(PartQ &p, float lo) {
-    p.mq += __float2int_rn(lo * kMassScale);
+    p.mq += __float2ll_rn(lo * kMassScale);
 }
 
 // A wetted cell's surface element and cos θ (surfacearea!, src/measures.jl).
