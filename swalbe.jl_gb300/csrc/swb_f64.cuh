@@ -260,20 +260,33 @@ __device__ __forceinline__ void relax64(O &o, const double fe[9], const double f
 // A Float64 value as an integer in units of 2^-96, split into four chunks of
 // 27 bits and a signed top chunk, so that a warp adds each chunk with one
 // 32-bit reduction: sums of these are exact and do not depend on their order.
-// Values from 2^30 on (and non-finite ones) are not held (false); bits below
-// 2^-96 are dropped.
+// Held are zeros and values from 2^-44 (whose last bit is 2^-96) up to 2^30;
+// of others the result is false.
 __device__ __forceinline__ bool chunks64(double v, uint32_t c[kChunks]) {
     const int e = (int)((hi64(v) >> 20) & 0x7ff) - 979;  // v = m 2^e in units of 2^-96
-    if (e > 73) return false;
-    const uint64_t m = e > -979 ? (__double_as_longlong(v) & 0xfffffffffffffull) | 0x10000000000000ull : 0ull;
-    unsigned __int128 u = e >= 0 ? (unsigned __int128)m << e : (unsigned __int128)(e > -64 ? m >> -e : 0);
+    const bool in = (uint32_t)e <= 73u;
+    if (!in && !zero64(v)) return false;
+    const uint64_t m = (__double_as_longlong(v) & 0xfffffffffffffull) | 0x10000000000000ull;
+    unsigned __int128 u = in ? (unsigned __int128)m << e : (unsigned __int128)0;
     if (hi64(v) & 0x80000000u) u = ~u + 1;
 #pragma unroll
     for (int i = 0; i < kChunks - 1; ++i) c[i] = (uint32_t)(u >> (27 * i)) & 0x7ffffffu;
     c[kChunks - 1] = (uint32_t)(int32_t)((__int128)u >> 108);
     return true;
 }
-// The value of chunk sums (each the sum of up to 2^31 chunks).
+// An integer as a double, rounded once.
+__device__ __forceinline__ double round128(__int128 u) {
+    const unsigned __int128 m = u < 0 ? -(unsigned __int128)u : (unsigned __int128)u;
+    const uint64_t h = (uint64_t)(m >> 64), l = (uint64_t)m;
+    double v = (double)l;
+    if (h) {  // the upper 64 bits, the last one sticky
+        const int s = 64 - __clzll((long long)h);
+        v = (double)((uint64_t)(m >> s) | ((m & (((unsigned __int128)1 << s) - 1)) ? 1u : 0u));
+        v *= __longlong_as_double((long long)(1023 + s) << 52);
+    }
+    return u < 0 ? -v : v;
+}
+// The value of chunk sums (each the sum of up to 2^31 chunks), rounded once.
 __device__ __forceinline__ double value64(const long long c[kChunks]) {
     long long d[kChunks], carry = 0;
 #pragma unroll
@@ -288,8 +301,7 @@ __device__ __forceinline__ double value64(const long long c[kChunks]) {
     const __int128 low = ((__int128)d[1] << 27) | d[0], mid = ((__int128)d[3] << 27) | d[2];
     const __int128 u = whole ? ((__int128)d[4] << 108) + (mid << 54) + low
                              : ((__int128)d[4] << 54) + (mid | (low ? 1 : 0));
-    const double v = (double)(long long)(u >> 64) * 0x1p64 + (double)(unsigned long long)u;
-    return v * (whole ? 0x1p-96 : 0x1p-42);
+    return round128(u) * (whole ? 0x1p-96 : 0x1p-42);
 }
 
 // Order-preserving keys for unsigned 64-bit maxima; 0 stands for no cell and

@@ -133,8 +133,12 @@ constexpr int kChunks = 5;                // integers a Float64 sum is split int
 constexpr int kSums64 = 3 * kChunks + 1;  // mass, area, cos-sum, wetted count
 constexpr int kLanes64 = 16;
 // accumulators of one iteration parity: sums, hmax and hmin keys, each in
-// kLanes64 lanes, then the Float64 sums of values the integers do not hold
-constexpr int kAcc64 = (kSums64 + 2) * kLanes64 + 4;
+// kLanes64 lanes, then of the mass, area and cos-sum what these integers do not
+// hold: a word that is not zero where there is any, the Float64 sums of values
+// that are not finite, and the limbs of the others (wide_add)
+constexpr int kWide64 = 68;
+constexpr int kOut64 = (kSums64 + 2) * kLanes64;
+constexpr int kAcc64 = kOut64 + 4 + 3 * kWide64;
 struct Cell64 {
     Fma64 f;
     double *p;                // film pressure of the iteration

@@ -119,9 +119,76 @@ __global__ void __launch_bounds__(kCellNT) cell_pressure_kernel(const StepArgs a
     x.p[c] = cell_pressure(a, x, h[c], near_cell(h, g), kap);
 }
 
+// Sums of values that chunks64 does not hold, over the whole range of Float64:
+// limb i of a sum counts units of 2^(32 i - 1074) in 64 bits, so that it takes
+// 2^31 values before it has to pass anything on, and the sum is exact and free
+// of order like the other.  (Rare, so one atomic per limb and value will do.)
+__device__ __forceinline__ void wide_add(unsigned long long *w, double v) {
+    const int e = (int)((hi64(v) >> 20) & 0x7ff), p = e ? e - 1 : 0;
+    const uint64_t m = (__double_as_longlong(v) & 0xfffffffffffffull) | (e ? 0x10000000000000ull : 0ull);
+    const unsigned __int128 u = (unsigned __int128)m << (p & 31);
+    const bool neg = hi64(v) & 0x80000000u;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const unsigned long long l = (uint32_t)(u >> (32 * i));
+        if (l) atomicAdd(w + p / 32 + i, neg ? 0ull - l : l);
+    }
+}
+// The value of the limbs w and chunk sums c together, rounded once; clears w.
+// One thread, with nobody else at w.
+__device__ __noinline__ double wide_value(unsigned long long *w, const long long *c) {
+    auto at = [&](int i) { return i < 0 ? 0ll : (long long)__ldcg(w + i); };
+    for (int i = 0; i < kChunks; ++i) {  // chunk i counts units of 2^(27 i - 96)
+        const int p = 27 * i + 1074 - 96;
+        const __int128 v = (__int128)c[i] << (p & 31);
+        w[p / 32] = (unsigned long long)(at(p / 32) + (long long)(uint32_t)v);
+        w[p / 32 + 1] = (unsigned long long)(at(p / 32 + 1) + (long long)(uint32_t)(v >> 32));
+        w[p / 32 + 2] = (unsigned long long)(at(p / 32 + 2) + (long long)(v >> 64));
+    }
+    long long carry = 0;
+    for (int i = 0; i < kWide64; ++i) {
+        const long long v = at(i) + carry;
+        w[i] = (uint32_t)v;
+        carry = v >> 32;
+    }
+    const bool neg = carry < 0;
+    if (neg) {  // the magnitude
+        carry = 1;
+        for (int i = 0; i < kWide64; ++i) {
+            const long long v = (long long)(uint32_t)~(uint32_t)at(i) + carry;
+            w[i] = (uint32_t)v;
+            carry = v >> 32;
+        }
+    }
+    int n = kWide64 - 1;
+    while (n >= 0 && !at(n)) --n;
+    double v = 0.0;
+    if (n >= 0) {  // the upper 64 bits, the last one sticky
+        const uint64_t h = (uint64_t)at(n) << 32 | (uint64_t)at(n - 1), l = (uint64_t)at(n - 2) << 32;
+        const int z = __clzll((long long)h);
+        uint64_t top = z ? h << z | l >> (64 - z) : h;
+        bool rest = (l << z) != 0;
+        for (int i = n - 3; i >= 0; --i) rest |= at(i) != 0;
+        if (rest) top |= 1;
+        v = ldexp((double)top, 32 * (n - 1) - z - 1074);
+    }
+    for (int i = 0; i < kWide64; ++i) w[i] = 0ull;
+    return neg ? -v : v;
+}
+
+__device__ __noinline__ void cell_measure_outside(unsigned long long *acc, int at, double v) {
+    unsigned long long *out = acc + kOut64;
+    out[0] = 1ull;
+    if (finite64(v))
+        wide_add(out + 4 + at * kWide64, v);
+    else
+        atomicAdd(reinterpret_cast<double *>(out) + 1 + at, v);
+}
+
 // The measures of an iteration's height: every warp adds its cells' values
 // as integers (chunks64: exact, in any order), the block its warps', and one
-// atomic per value adds the block's to lane blockIdx % kLanes64.
+// atomic per value adds the block's to lane blockIdx % kLanes64.  Values that
+// chunks64 does not hold are added one by one, exactly as well.
 template <int NT>
 __device__ __forceinline__ void cell_measures(const StepArgs &a, const Cell64 &x, int par, bool in,
                                               double h, double area, double cs, bool wet) {
@@ -129,7 +196,6 @@ __device__ __forceinline__ void cell_measures(const StepArgs &a, const Cell64 &x
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const bool with_area = a.meas_mask & SWB_MEAS_AREA;
     unsigned long long *acc = x.acc + (size_t)par * kAcc64;
-    double *big = reinterpret_cast<double *>(acc + kSums64 * kLanes64 + 2 * kLanes64);
     uint32_t ch[kChunks];
     auto add = [&](double v, bool on, int at) {
 #pragma unroll
@@ -137,7 +203,7 @@ __device__ __forceinline__ void cell_measures(const StepArgs &a, const Cell64 &x
         if (on && !chunks64(v, ch)) {
 #pragma unroll
             for (int q = 0; q < kChunks; ++q) ch[q] = 0;
-            atomicAdd(big + at, v);
+            cell_measure_outside(acc, at, v);
         }
 #pragma unroll
         for (int q = 0; q < kChunks; ++q) {
@@ -189,7 +255,6 @@ __device__ void cell_reduce(const StepArgs &a, const Cell64 &x, long long s) {
     __shared__ long long sum[kSums64];
     __shared__ unsigned long long mx[2];
     unsigned long long *acc = x.acc + (size_t)(s & 1) * kAcc64;
-    double *big = reinterpret_cast<double *>(acc + kSums64 * kLanes64 + 2 * kLanes64);
     const int lane = threadIdx.x & (kLanes64 - 1), grp = threadIdx.x / kLanes64;
     constexpr int G = NT / kLanes64;  // fields handled at a time
     static_assert(kLanes64 == 16 && (kSums64 + 2) % 2 == 0, "half-warp reductions");
@@ -214,13 +279,16 @@ __device__ void cell_reduce(const StepArgs &a, const Cell64 &x, long long s) {
     __syncthreads();
     if (threadIdx.x == 0) {
         double v[3];
-        for (int q = 0; q < 3; ++q) {
-            v[q] = value64(sum + q * kChunks);
-            const double b = __ldcg(big + q);
-            if (b != 0.0) {
-                v[q] += b;
-                big[q] = 0.0;
+        unsigned long long *out = acc + kOut64;
+        if (__ldcg(out)) {
+            double *inf = reinterpret_cast<double *>(out) + 1;
+            for (int q = 0; q < 3; ++q) {
+                v[q] = wide_value(out + 4 + q * kWide64, sum + q * kChunks) + __ldcg(inf + q);
+                inf[q] = 0.0;
             }
+            out[0] = 0ull;
+        } else {
+            for (int q = 0; q < 3; ++q) v[q] = value64(sum + q * kChunks);
         }
         finish_step(a, s, v[0], (double)sum[kSums64 - 1], mx[0] ? unorder64(mx[0]) : -INFINITY,
                     mx[1] ? unorder64(~mx[1]) : INFINITY, v[1], v[2]);
