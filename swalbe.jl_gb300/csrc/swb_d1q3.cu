@@ -357,12 +357,12 @@ __global__ void __launch_bounds__(kD1Halves<R> * NT) d1q3_run_kernel(const D1Arg
 }
 
 // The records of n iterations after t0 from their warps' measures: one warp
-// per lattice (blockIdx.y) and iteration.
+// per lattice (blockIdx.x, of which there may be more than 65535) and iteration.
 __global__ void __launch_bounds__(128) d1q3_record_kernel(const D1Args *__restrict__ args,
                                                           const D1Part *__restrict__ part, int nchunks,
                                                           int warps, int n, long long t0) {
-    const D1Args &a = args[blockIdx.y];
-    const int k = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const D1Args &a = args[blockIdx.x];
+    const int k = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (k >= n || !a.rec || n - k > a.rec_cap) return;  // only the newest the ring holds
     long long c[kChunks] = {};
     unsigned long long mx = 0, mn = 0;
@@ -773,7 +773,7 @@ int swb1d_step(swb1d *b, int64_t nsteps) {
             done += n;
         }
         if (b->rec_cap) {
-            swb::d1q3_record_kernel<<<dim3((unsigned)((burst + 3) / 4), (unsigned)b->count), 128, 0, b->stream>>>(
+            swb::d1q3_record_kernel<<<dim3((unsigned)b->count, (unsigned)((burst + 3) / 4)), 128, 0, b->stream>>>(
                 b->d_args, b->d_part, b->nchunks, warps, burst, b->t);
             swb::count_launches(1);
             D1_TRY(b, cudaGetLastError());
