@@ -26,6 +26,7 @@
 #include <cstdint>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "swb_f64.cuh"
@@ -77,41 +78,57 @@ struct D1Cell {
 };
 template <class R>
 struct D1Mid {
-    R slip, fe[3];
+    R slip, half, fe[3];  // slippage, h / 2, equilibrium
 };
 
-// One cell's operations, Float64: rounded as the reference's, with products by
-// powers of two inside the sum that follows them (exact, short of subnormal
-// numbers).
+// One cell's operations, Float64: rounded as the reference's.  With g = 0 and
+// τ = 1 the products with 0 are left out, which are zeros unless a factor is not
+// finite: such cells are computed again with Plain64, which leaves nothing out.
 template <class O>
 struct D1Cell64 {
+    static constexpr bool kPlain = std::is_same<O, Plain64>::value;
     O o;
+    __device__ __forceinline__ static double or_nan(double v, double factor) {
+        return finite64(factor) ? v : __longlong_as_double(0x7ff8000000000000LL);
+    }
     __device__ __forceinline__ double quot(double a, double b) { return o.quot(a, b, o.recip(b)); }
     __device__ __forceinline__ double pressure(const D1Args &a, const D1Cell<double> &c, double h, double hip,
                                                double him) {
         double pn, pm;
         powers64(o, quot(a.hmin, o.add(h, a.hcrit)), a.n, a.m, pn, pm);
         const double p = o.mul(-c.gam, o.mul(c.kap, o.sub(pn, pm)));
-        return o.sub(p, o.mul(c.gam, o.add(o.twice_plus(-h, hip), him)));
+        return o.sub(p, o.mul(c.gam, o.add(o.twice_plus(large64(-h), hip), him)));
     }
     // slippage and equilibrium, which need only the cell's own fields
-    __device__ __forceinline__ void local(const D1Cell<double> &c, double h, double u, D1Mid<double> &m) {
-        const double den = o.add(o.twice_plus(o.muln(h, h), o.mul(c.delta6, h)), c.delta3sq);
+    __device__ __forceinline__ void local(const D1Cell<double> &c, double h, double u, const double fo[3],
+                                          D1Mid<double> &m) {
+        const double den = o.add(o.twice_plus(large64(o.muln(h, h)), o.mul(c.delta6, h)), c.delta3sq);
         m.slip = quot(o.mul(o.mul(c.mu6, h), u), den);
-        const double uu = o.mul(u, u);
-        const double gh = c.g == 0.0 ? 0.0 : o.muln(c.g25, h);
-        m.fe[0] = o.muln(h, o.sub(c.g == 0.0 ? 1.0 : o.sub(1.0, o.muln(c.g50, h)), uu));
-        m.fe[1] = o.mul(h, __fma_rn(0.5, uu, __fma_rn(0.5, u, gh)));
-        m.fe[2] = o.mul(h, __fma_rn(0.5, uu, __fma_rn(-0.5, u, gh)));
+        m.half = half64(h);
+        const double uu = o.mul(u, u), u2 = half64(u), uu2 = half64(uu);
+        if (c.g == 0.0 && !kPlain) {
+            m.fe[0] = o.muln(h, o.sub(1.0, uu));
+            m.fe[1] = o.mul(h, o.add(u2, uu2));
+            m.fe[2] = o.mul(h, o.sub(uu2, u2));
+        } else {
+            const double gh = o.muln(c.g25, h);
+            m.fe[0] = o.muln(h, o.sub(o.sub(1.0, o.muln(c.g50, h)), uu));
+            m.fe[1] = o.mul(h, o.add(o.add(gh, u2), uu2));
+            m.fe[2] = o.mul(h, o.add(o.sub(gh, u2), uu2));
+        }
+        if (c.tau1 && kPlain)  // 0 fo
+#pragma unroll
+            for (int q = 0; q < 3; ++q) m.fe[q] = or_nan(m.fe[q], fo[q]);
     }
-    __device__ __forceinline__ void second(const D1Cell<double> &c, double h, const D1Mid<double> &m, double pm,
-                                           double pp, const double fo[3], double out[3]) {
-        double F = __fma_rn(0.5, o.mul(h, o.sub(pm, pp)), -m.slip);
+    __device__ __forceinline__ void second(const D1Cell<double> &c, const D1Mid<double> &m, double pm, double pp,
+                                           const double fo[3], double out[3]) {
+        double F = o.sub(o.mul(m.half, o.sub(pm, pp)), m.slip);
         if (c.grad) F = o.sub(F, c.dg);
         double fe[3] = {m.fe[0], m.fe[1], m.fe[2]};
         if (!c.tau1)
 #pragma unroll
             for (int q = 0; q < 3; ++q) fe[q] = o.add(o.mul(c.omeg, fo[q]), o.mul(c.invtau, fe[q]));
+        F = even64(F);
         out[0] = fe[0];
         out[1] = __fma_rn(0.5, F, fe[1]);
         out[2] = __fma_rn(-0.5, F, fe[2]);
@@ -127,12 +144,13 @@ __device__ __noinline__ double d1_pressure_again(const D1Args &a, const D1Cell<d
                                                  double him) {
     return D1Cell64<Plain64>{}.pressure(a, c, h, hip, him);
 }
-__device__ __noinline__ void d1_local_again(const D1Cell<double> &c, double h, double u, D1Mid<double> *m) {
-    D1Cell64<Plain64>{}.local(c, h, u, *m);
+__device__ __noinline__ void d1_local_again(const D1Cell<double> &c, double h, double u, const double *fo,
+                                            D1Mid<double> *m) {
+    D1Cell64<Plain64>{}.local(c, h, u, fo, *m);
 }
-__device__ __noinline__ void d1_second_again(const D1Cell<double> &c, double h, const D1Mid<double> &m, double pm,
-                                             double pp, const double *fo, double *out) {
-    D1Cell64<Plain64>{}.second(c, h, m, pm, pp, fo, out);
+__device__ __noinline__ void d1_second_again(const D1Cell<double> &c, const D1Mid<double> &m, double pm, double pp,
+                                             const double *fo, double *out) {
+    D1Cell64<Plain64>{}.second(c, m, pm, pp, fo, out);
 }
 __device__ __noinline__ void d1_moments_again(const double *f, double *h, double *u) {
     D1Cell64<Plain64>{}.moments(f, *h, *u);
@@ -157,26 +175,29 @@ struct D1Ops64 {
         const D1Cell<double> cc = c;
         return d1_pressure_again(a, cc, h, hip, him);
     }
-    __device__ __forceinline__ void local(const D1Cell<double> &c, double h, double u, D1Mid<double> &m) const {
+    // odd: the height or a population is not finite
+    __device__ __forceinline__ void local(const D1Cell<double> &c, double h, double u, const double fo[3], bool odd,
+                                          D1Mid<double> &m) const {
         D1Cell64<FAST> k{FAST(f)};
-        k.local(c, h, u, m);
-        if (k.o.bad) {
+        k.local(c, h, u, fo, m);
+        if (k.o.bad | odd) {
             const D1Cell<double> cc = c;
+            const double in[3] = {fo[0], fo[1], fo[2]};
             D1Mid<double> again;
-            d1_local_again(cc, h, u, &again);
+            d1_local_again(cc, h, u, in, &again);
             m = again;
         }
     }
-    __device__ __forceinline__ void second(const D1Cell<double> &c, double h, const D1Mid<double> &m, double pm,
+    __device__ __forceinline__ void second(const D1Cell<double> &c, double, const D1Mid<double> &m, double pm,
                                            double pp, const double fo[3], double out[3]) const {
         D1Cell64<FAST> k{FAST(f)};
-        k.second(c, h, m, pm, pp, fo, out);
+        k.second(c, m, pm, pp, fo, out);
         if (k.o.bad) {
             const D1Cell<double> cc = c;
             const D1Mid<double> mm = m;
             const double in[3] = {fo[0], fo[1], fo[2]};
             double again[3];
-            d1_second_again(cc, h, mm, pm, pp, in, again);
+            d1_second_again(cc, mm, pm, pp, in, again);
 #pragma unroll
             for (int q = 0; q < 3; ++q) out[q] = again[q];
         }
@@ -208,7 +229,8 @@ struct D1Ops32 {
         const float p = -c.gam * (c.kap * (pow_n(x, a.n) - pow_n(x, a.m)));
         return p - c.gam * ((hip - 2.0f * h) + him);
     }
-    __device__ __forceinline__ void local(const D1Cell<float> &c, float h, float u, D1Mid<float> &m) const {
+    __device__ __forceinline__ void local(const D1Cell<float> &c, float h, float u, const float *, bool,
+                                          D1Mid<float> &m) const {
         m.slip = (c.mu6 * h * u) / ((2.0f * (h * h) + c.delta6 * h) + c.delta3sq);
         const float uu = u * u;
         m.fe[0] = h * ((1.0f - (0.5f * c.g) * h) - uu);
@@ -310,6 +332,7 @@ __global__ void __launch_bounds__(kD1Halves<R> * NT) d1q3_run_kernel(const D1Arg
     const R *ff = reinterpret_cast<const R *>(a.f[from]);
     R h = reinterpret_cast<const R *>(a.h[from])[g], u = reinterpret_cast<const R *>(a.u[from])[g];
     R fo[3] = {ff[g], ff[L + g], ff[2 * L + g]}, p = R(0);
+    bool odd = !(finite(h) && finite(fo[0]) && finite(fo[1]) && finite(fo[2]));
     int bad = 0;
 #pragma unroll 1
     for (int k = 0; k < n; ++k) {
@@ -327,7 +350,7 @@ __global__ void __launch_bounds__(kD1Halves<R> * NT) d1q3_run_kernel(const D1Arg
                            hc > R(0.055));
         }
         if (second && in) {
-            op.local(c, h, u, m);
+            op.local(c, h, u, fo, odd, m);
         }
         __syncthreads();
         R o[3];
@@ -342,7 +365,8 @@ __global__ void __launch_bounds__(kD1Halves<R> * NT) d1q3_run_kernel(const D1Arg
             fo[1] = s1[tm];
             fo[2] = s2[tp];
             op.moments(fo, h, u);
-            if (own && !finite(h)) bad = 1;
+            odd = !finite(h);  // as it is where a population is not
+            if (own && odd) bad = 1;
         }
     }
     if (!own) return;

@@ -17,11 +17,34 @@ __device__ __forceinline__ uint32_t hi64(double v) { return (uint32_t)__double2h
 __device__ __forceinline__ uint32_t lo64(double v) { return (uint32_t)__double2loint(v); }
 __device__ __forceinline__ bool finite64(double v) { return (hi64(v) & 0x7ff00000u) != 0x7ff00000u; }
 
+__device__ __forceinline__ bool zero64(double v) { return ((hi64(v) & 0x7fffffffu) | lo64(v)) == 0; }
+// v / 2 by its exponent, on the Float64 unit only where that is not enough (an asm
+// statement, which is not computed beside the other case and then selected).
+__device__ __forceinline__ double half64(double v) {
+    if (((hi64(v) >> 20) & 0x7ff) - 2u <= 2044u) return __hiloint2double((int)(hi64(v) - 0x100000u), (int)lo64(v));
+    asm volatile("mul.rn.f64 %0, %0, 0d3FE0000000000000;" : "+d"(v));
+    return v;
+}
+
+// v, but where v / 2 is rounded (v below 2^-1021) the number twice as large as
+// that, and where 2 v overflows infinity: 0.5 even64(v) + b and 2 large64(v) + b
+// as one fused operation round as the two they stand for.  (Selections of a few
+// integer instructions; a branch costs a warp alone on its SM quarter 20 to 70 ns.)
+__device__ __forceinline__ double even64(double v) {
+    const uint32_t h = hi64(v), l = lo64(v);
+    const long long odd = ((h & 0x7fe00000u) == 0u && (l & 1u)) ? (long long)(int)(l & 2u) - 1 : 0;
+    return __longlong_as_double(__double_as_longlong(v) + odd);
+}
+__device__ __forceinline__ double large64(double v) {
+    const bool big = (hi64(v) & 0x7ff00000u) == 0x7fe00000u;
+    return __hiloint2double((int)(big ? (hi64(v) | 0x7ff00000u) & 0xfff00000u : hi64(v)),
+                            (int)(big ? 0u : lo64(v)));
+}
+
 // a b rounded to nearest, of normal numbers or (ZERO) zeros, in integers: the
 // 106-bit product of the significands, its upper 62 or 63 bits with a sticky
 // last bit, rounded half to even at bit 10.  Sets `bad` where an operand or
 // the result is neither: the caller then computes the cell again (Plain64).
-__device__ __forceinline__ bool zero64(double v) { return ((hi64(v) & 0x7fffffffu) | lo64(v)) == 0; }
 template <bool ZERO>
 __device__ __forceinline__ double mul64(double a, double b, bool &bad) {
     const uint32_t ah = hi64(a), bh = hi64(b);
@@ -109,7 +132,7 @@ __device__ __forceinline__ double quot64(double a, double b, uint64_t r, bool &b
 
 // The operations of a cell.  mul: operands that may be zero; muln: operands
 // that are not (a zero is then computed again); twice_plus: 2 a + b, rounded
-// once either way because 2 a is exact.
+// once either way because 2 a is exact (or, beyond large64, infinite).
 struct Fast64 {
     Fma64 f;
     bool bad;
