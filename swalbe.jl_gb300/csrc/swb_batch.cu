@@ -344,10 +344,11 @@ int autotune(swb_batch *b, long long &left) {
             for (const swb_params &p : b->params) sizes.push_back({p.Lx, p.Ly});
             std::vector<std::tuple<double, int, int>> est;
             for (int nt : {-64, -32}) {
+                const swb::StripColumns columns = swb::strip_columns(sizes, swb::pair_columns(nt));
                 const int slots = swb::batch_blocks_per_sm(b->precision, nt, wave);
                 double last = -1.0;
                 for (int cap = 64; cap >= swb::kMinRows; --cap) {
-                    const double us = swb::pair_iteration_us(sizes, nt, cap, sms, slots);
+                    const double us = swb::pair_iteration_us(columns, nt, cap, sms, slots);
                     if (us != last) est.push_back({us, nt, cap});
                     last = us;
                 }

@@ -5,6 +5,7 @@
 
 #include <cmath>
 #include <string>
+#include <unordered_map>
 #include <utility>
 #include <vector>
 
@@ -60,8 +61,21 @@ inline int balanced_rows(int Ly, int cap) {
     const int strips = (Ly + cap - 1) / cap;
     return (Ly + strips - 1) / strips;
 }
-// Estimated time of an iteration of many lattices (Lx, Ly) on pair strips of
-// geometry nt and at most cap rows, balanced: launch and drain, then waves of
+// Lattices (Lx, Ly) cut into strips of w columns, by height: (Ly, column strips of
+// all lattices that high).  An estimate is made for each of up to 126 strip sizes
+// whenever a server's resident set changes, and takes a pass over the heights
+// instead of the lattices (a server's 3000 requests of 32 to 64 columns and rows
+// that join and leave: 0.51 s with passes over the lattices, 0.32 s so).
+using StripColumns = std::vector<std::pair<int, double>>;
+inline StripColumns strip_columns(const std::vector<std::pair<int, int>> &sizes, int w) {
+    std::unordered_map<int, double> of;
+    for (const auto &p : sizes) of[p.second] += (double)((p.first + w - 1) / w);
+    return StripColumns(of.begin(), of.end());
+}
+// Columns of the pair strips of geometry nt.
+inline int pair_columns(int nt) { return -2 * nt - 4; }
+// Estimated time of an iteration of many lattices on pair strips of geometry nt
+// and at most cap rows, balanced: launch and drain, then waves of
 // up to `slots` CTAs per SM, each as long as a march over the tallest strip.
 // c CTAs of 64 threads (or 2 c of 32) on an SM take 0.655 us per row up to
 // c = 1.4 and 0.11 us more for each further one.  Measured on GB300 with the θ
@@ -69,14 +83,13 @@ inline int balanced_rows(int Ly, int cap) {
 // within 20 % of all, and the strips it picks within 15 % of the best.  E.g. a
 // 1024² lattice 50.7 us with 64 rows, 21.0 with 8; eight of 32k to 147k cells
 // 51.1 and 17.7 (60 columns, 6 rows).
-inline double pair_iteration_us(const std::vector<std::pair<int, int>> &sizes, int nt, int cap, int sms, int slots) {
-    const int w = -2 * nt - 4;
+inline double pair_iteration_us(const StripColumns &columns, int nt, int cap, int sms, int slots) {
     double strips = 0.0;
     int tallest = 0;
-    for (const auto &p : sizes) {
-        const int h = balanced_rows(p.second, cap);
+    for (const auto &p : columns) {
+        const int h = balanced_rows(p.first, cap);
         tallest = h > tallest ? h : tallest;
-        strips += (double)((p.first + w - 1) / w) * (double)((p.second + h - 1) / h);
+        strips += p.second * (double)((p.first + h - 1) / h);
     }
     const double c = strips / sms, waves = std::floor(c / slots), rest = c - slots * waves;
     auto row = [nt](double c) { return 0.655 * (1.0 + 0.17 * std::fmax(0.0, c * (-nt / 64.0) - 1.4)); };

@@ -188,24 +188,24 @@ constexpr int kServePairRows = 64;
 // Estimated time of an iteration of the resident set.  Pair strips:
 // pair_iteration_us.  One-column strips: the march of the tallest at 0.6 us per
 // row (Float64: 10), or 55 cells per ns (2).
-double iteration_us(const swb_server *sv, int nt, int cap, int sms, int slots) {
-    std::vector<std::pair<int, int>> sizes;
-    for (const Req *r : sv->active) sizes.push_back({r->p.Lx, r->p.Ly});
-    if (nt < 0) return swb::pair_iteration_us(sizes, nt, cap, sms, slots);
+double iteration_us(const swb_server *sv, const swb::StripColumns &columns, int nt, int cap, int sms, int slots) {
+    if (nt < 0) return swb::pair_iteration_us(columns, nt, cap, sms, slots);
     const bool f64 = sv->precision == SWB_F64;
     double cells = 0.0;
     int tallest = 0;
-    for (const auto &p : sizes) {
-        const int h = swb::balanced_rows(p.second, cap), w = nt - 4;
+    for (const auto &p : columns) {
+        const int h = swb::balanced_rows(p.first, cap);
         tallest = std::max(tallest, h);
-        cells += (double)((p.first + w - 1) / w) * nt * (double)((p.second + h - 1) / h) * (h + 4);
+        cells += p.second * nt * (double)((p.first + h - 1) / h) * (h + 4);
     }
     return std::max((tallest + 4) * (f64 ? 10.0 : 0.6), cells / (f64 ? 2e3 : 55e3));
 }
 void choose_geometry(swb_server *sv, int sms) {
     bool pair = sv->precision == SWB_F32 || sv->precision == SWB_F16;
     bool wave = false;
+    std::vector<std::pair<int, int>> sizes;
     for (Req *r : sv->active) {
+        sizes.push_back({r->p.Lx, r->p.Ly});
         pair = pair && r->p.Lx % 2 == 0 && swb::pair_form_ok(r->a);
         wave = wave || r->a.theta_mode == swb::THETA_WAVE;
     }
@@ -214,9 +214,10 @@ void choose_geometry(swb_server *sv, int sms) {
     for (int nt : {-64, -32, swb::kBatchNT}) {
         if ((nt < 0) != pair || (pair && sv->geo_nt != 0 && nt != sv->geo_nt)) continue;
         const int slots = pair ? swb::batch_blocks_per_sm(sv->precision, nt, wave) : 0;
+        const swb::StripColumns columns = swb::strip_columns(sizes, pair ? swb::pair_columns(nt) : nt - 4);
         for (int k = pair ? kServePairRows : swb::kBatchRows; k >= swb::kMinRows; --k) {
             const int cap = pair && sv->geo_rows > 0 ? sv->geo_rows : k;
-            const double us = iteration_us(sv, nt, cap, sms, slots);
+            const double us = iteration_us(sv, columns, nt, cap, sms, slots);
             if (best < 0.0 || us < best) {
                 best = us;
                 best_nt = nt;
