@@ -605,8 +605,8 @@ int run_grid(swb_state *s) {
 }
 
 // Whether the state's iterations can run in its multi-step form now:
-// strips / 2D tiles of FP32-arithmetic states, or resident tiles for the
-// common steady τ = 1 step.
+// strips / 2D tiles of FP32-arithmetic states, or resident tiles for
+// steady τ = 1 steps.
 bool run_possible(const swb_state *s) {
     if (s->precision != SWB_F32 && s->precision != SWB_F16) return false;
     if (swb::resident_geometry(s->a.march_nt))

@@ -174,8 +174,8 @@ inline bool pair_geometry(int nt) { return nt == -32 || nt == -64 || nt == -128;
 // Resident tiles (a multi-step launch form, SWB_F32 / SWB_F16): geometry
 // value kResGeom, tiles of kResTW columns x h rows (1 <= h <= kResMaxTH), one
 // CTA of kResThreads threads per tile holding the tile's populations in
-// shared memory, all CTAs co-resident.  Only the common steady τ = 1 step
-// has this form; other iterations run on strips (strip_fallback).
+// shared memory, all CTAs co-resident.  Steady τ = 1 steps have this form
+// (resident_ok); other iterations run on strips (strip_fallback).
 constexpr int kResGeom = 33;
 // kResGeom2: the same with CTAs of kResThreads / 2 threads, two per SM (one
 // CTA's phases run while the other waits at a barrier; tiles half as tall).

@@ -493,7 +493,9 @@ __device__ __forceinline__ void mass_add(PartQ &p, float v) {
 }
 
 // The rounding residue of a cell's pulled height (up to half an ulp of h: 0.5 and
-// more, which 32 bits would not hold, from heights of 2^23 on).
+// more, which 32 bits would not hold, from heights of 2^23 on; the 32-bit conversion
+// alone would save 0.5 us of 53.4 at 2048² FP32, 0.8 of 49.6 with FP16 storage, and
+// both with a branch cost 53.7 and 50.4).
 template <class R>
 __device__ __forceinline__ void mass_add_lo(PartT<R> &p, R lo) { p.mlo = p.mlo + lo; }
 __device__ __forceinline__ void mass_add_lo(PartQ &p, float lo) {
