@@ -58,6 +58,23 @@ __device__ __forceinline__ T *at(T *plane, int i) {
     return reinterpret_cast<T *>(reinterpret_cast<char *>(plane) + (unsigned)i * (unsigned)sizeof(T));
 }
 
+// Where a kernel loads from and stores to: by such offsets or as an array.  (The
+// order of the additions is part of what the compiler makes of it.)
+template <bool OFFSETS, class T>
+__device__ __forceinline__ const T *load_from(const T *b, int plane, int i) {
+    if constexpr (OFFSETS)
+        return at(b + plane, i);
+    else
+        return b + plane + i;
+}
+template <bool OFFSETS, class T>
+__device__ __forceinline__ T &store_to(T *b, int plane, int i) {
+    if constexpr (OFFSETS)
+        return *at(b + plane, i);
+    else
+        return b[plane + i];
+}
+
 template <class L>
 struct StoreF64T {
     using real = double;
@@ -71,24 +88,26 @@ struct StoreF64T {
     }
 };
 
-template <class L>
+// OFFSETS: byte offsets from the planes' addresses (at), see StripStore.
+template <class L, bool OFFSETS = false>
 struct StoreF32T {
     using real = float;
     static constexpr bool kLiteral = false;
     static constexpr bool kHalf = false;
     __device__ __forceinline__ static float ld(const void *b, int pitch, int q, int i) {
-        return L::ld(at(reinterpret_cast<const float *>(b) + q * pitch, i));
+        return L::ld(load_from<OFFSETS>(reinterpret_cast<const float *>(b), q * pitch, i));
     }
     __device__ __forceinline__ static void st(void *b, int pitch, int q, int i, float v) {
-        *at(reinterpret_cast<float *>(b) + q * pitch, i) = v;
+        store_to<OFFSETS>(reinterpret_cast<float *>(b), q * pitch, i) = v;
     }
 };
 
 // f0 as an FP32 plane, f1..f8 as FP16 planes holding 2^10 f_q (the scale
 // keeps populations of order 1e-5..1e-2 in the normal FP16 range).
-template <class L>
+template <class L, bool OFFSETS = true>
 struct StoreF16T {
     using real = float;
+    static constexpr bool kOffsets = OFFSETS;
     static constexpr bool kLiteral = false;
     static constexpr bool kHalf = true;
     static constexpr float kScale = 1024.0f;
@@ -97,15 +116,15 @@ struct StoreF16T {
         return reinterpret_cast<const __half *>(reinterpret_cast<const float *>(b) + pitch);
     }
     __device__ __forceinline__ static float ld(const void *b, int pitch, int q, int i) {
-        if (q == 0) return L::ld(at(reinterpret_cast<const float *>(b), i));
-        return __half2float(L::ld(at(hp(b, pitch) + (q - 1) * pitch, i))) * kInv;
+        if (q == 0) return L::ld(load_from<OFFSETS>(reinterpret_cast<const float *>(b), 0, i));
+        return __half2float(L::ld(load_from<OFFSETS>(hp(b, pitch), (q - 1) * pitch, i))) * kInv;
     }
     __device__ __forceinline__ static void st(void *b, int pitch, int q, int i, float v) {
         if (q == 0) {
-            *at(reinterpret_cast<float *>(b), i) = v;
+            store_to<OFFSETS>(reinterpret_cast<float *>(b), 0, i) = v;
         } else {
             __half *h = const_cast<__half *>(hp(b, pitch));
-            *at(h + (q - 1) * pitch, i) = __float2half_rn(v * kScale);
+            store_to<OFFSETS>(h, (q - 1) * pitch, i) = __float2half_rn(v * kScale);
         }
     }
 };
@@ -113,6 +132,29 @@ struct StoreF16T {
 using StoreF64 = StoreF64T<LdNC>;
 using StoreF32 = StoreF32T<LdNC>;
 using StoreF16 = StoreF16T<LdNC>;
+
+// How the one-column strips of a single lattice address their planes.  Offsets
+// save instructions, but some forms need so many more registers with them that
+// fewer CTAs fit an SM: FP32 strips of 64 threads 80 instead of 64 (2047² with
+// 32 rows 60.0 us per iteration as arrays, 76.8 with offsets; τ = 0.8 85.9 and
+// 104), FP16 with rare forces or θ fields 126 instead of 96 (2047² 93.6 and 110),
+// and FP16 of 256 threads 126 instead of 80 (95.9 and 114).  Where they do not,
+// offsets are faster: FP32 with rare forces 126 either way (1001 x 1025 21.6 and
+// 20.4), other FP16 (2047² τ = 0.8 107 and 93.4).
+template <class S, bool GEN, int NT>
+struct StripStoreOf {
+    using type = S;
+};
+template <class L, bool GEN, int NT>
+struct StripStoreOf<StoreF32T<L>, GEN, NT> {
+    using type = StoreF32T<L, GEN>;
+};
+template <class L, bool GEN, int NT>
+struct StripStoreOf<StoreF16T<L>, GEN, NT> {
+    using type = StoreF16T<L, !GEN && NT < 256>;
+};
+template <class S, bool GEN, int NT>
+using StripStore = typename StripStoreOf<S, GEN, NT>::type;
 
 // ------------------------------------------------------------ launch overlap
 // Programmatic dependent launch.  The kernels of a step sequence (step,
@@ -1134,11 +1176,13 @@ __device__ __forceinline__ void collide_cell(const StepArgs &a,
         if constexpr (S::kHalf) {
             reinterpret_cast<float *>(dst)[cell] = fo[0];
             __half *hpl = const_cast<__half *>(S::hp(dst, pitch));
+            if (!S::kOffsets) hpl += cell;
+            const int c = S::kOffsets ? cell : 0;
             // planes 1..8 in the order of hb: (1, 2), (3, 4), (5, 6), (7, 8)
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                *at(hpl + (2 * k) * pitch, cell) = __low2half(hb[k]);
-                *at(hpl + (2 * k + 1) * pitch, cell) = __high2half(hb[k]);
+                store_to<S::kOffsets>(hpl, (2 * k) * pitch, c) = __low2half(hb[k]);
+                store_to<S::kOffsets>(hpl, (2 * k + 1) * pitch, c) = __high2half(hb[k]);
             }
         } else {
 #pragma unroll
@@ -2066,7 +2110,8 @@ enum StepForm { kFormAny = 0, kFormSteadyTau1 = 1, kFormSteady = 2 };
 // a reducer CTA, block 0, for the previous iteration's measures.
 template <class S, int NT, bool GEN, int FORM = kFormAny, bool WAVE = false>
 __global__ void __launch_bounds__(NT) fused_step_kernel(const StepArgs a, int k) {
-    __shared__ MarchSmem<S, NT> sm;
+    using P = StripStore<S, GEN, NT>;
+    __shared__ MarchSmem<P, NT> sm;
     grid_dep_wait();
     int b = blockIdx.x;
     if (needs_partials(a) && k > 0) {
@@ -2079,11 +2124,11 @@ __global__ void __launch_bounds__(NT) fused_step_kernel(const StepArgs a, int k)
     }
     const long long done = a.ctl->step_base + k;
     if constexpr (FORM == kFormSteadyTau1)
-        march_run<S, NT, false, true, GEN, WAVE>(a, b % a.tiles_x, b / a.tiles_x, done, sm);
+        march_run<P, NT, false, true, GEN, WAVE>(a, b % a.tiles_x, b / a.tiles_x, done, sm);
     else if constexpr (FORM == kFormSteady)
-        march_run<S, NT, false, false, GEN, WAVE>(a, b % a.tiles_x, b / a.tiles_x, done, sm);
+        march_run<P, NT, false, false, GEN, WAVE>(a, b % a.tiles_x, b / a.tiles_x, done, sm);
     else
-        march_tile<S, NT, GEN>(a, b % a.tiles_x, b / a.tiles_x, done, sm);
+        march_tile<P, NT, GEN>(a, b % a.tiles_x, b / a.tiles_x, done, sm);
 }
 
 // Closes a sequence of n step launches: the last iteration's measures, then
