@@ -356,10 +356,13 @@ int autotune(swb_batch *b, long long &left) {
             std::sort(est.begin(), est.end());
             for (size_t i = 0; i < est.size() && i < 4; ++i) geos.push_back({std::get<1>(est[i]), std::get<2>(est[i])});
         }
+        pair = !geos.empty();
         geos.push_back({64, 32});
         geos.push_back({64, 16});
+        if (!pair) geos.push_back({128, 16});
     }
-    const int probe = 4;
+    // pair strips of different numbers of rows differ by less than other strips do
+    const int probe = pair && !b->geometry_fixed ? 4 : 2;
     struct Best {
         float ms = 1e30f;
         int nt = 0, rows = 0, grid = 0;
