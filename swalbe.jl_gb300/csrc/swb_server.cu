@@ -210,7 +210,7 @@ void choose_geometry(swb_server *sv, int sms) {
         wave = wave || r->a.theta_mode == swb::THETA_WAVE;
     }
     int best_nt = swb::kBatchNT, best_cap = kServePairRows;
-    double best = -1.0;
+    double best = -1.0, tall = -1.0;
     for (int nt : {-64, -32, swb::kBatchNT}) {
         if ((nt < 0) != pair || (pair && sv->geo_nt != 0 && nt != sv->geo_nt)) continue;
         const int slots = pair ? swb::batch_blocks_per_sm(sv->precision, nt, wave) : 0;
@@ -218,6 +218,7 @@ void choose_geometry(swb_server *sv, int sms) {
         for (int k = pair ? kServePairRows : swb::kBatchRows; k >= swb::kMinRows; --k) {
             const int cap = pair && sv->geo_rows > 0 ? sv->geo_rows : k;
             const double us = iteration_us(sv, columns, nt, cap, sms, slots);
+            if (tall < 0.0) tall = us;  // of kBatchRows (one-column strips)
             if (best < 0.0 || us < best) {
                 best = us;
                 best_nt = nt;
@@ -225,6 +226,11 @@ void choose_geometry(swb_server *sv, int sms) {
             }
         }
     }
+    // the one-column estimate leaves out that CTAs per SM are whole numbers, so rows
+    // that promise less than 5 % are not taken (1023 x 1025 FP32: 27 rows promise 1 %
+    // and give 5 CTAs on the busiest SM for 4: 26.6 for 24.9 us per iteration; FP16
+    // is an exception, 37.5 for 42.1)
+    if (!pair && sv->precision != SWB_F16 && best > 0.95 * tall) best_cap = swb::kBatchRows;
     sv->nt = best_nt;
     for (Req *r : sv->active)
         swb::set_geometry(r->a, sv->nt, std::max(swb::balanced_rows(r->p.Ly, best_cap), swb::kMinRows));
