@@ -2148,11 +2148,23 @@ __global__ void __launch_bounds__(NT) advance_kernel(const StepArgs a, int n) {
 // entries with tx = -1 reduce their lattice's previous iteration.
 // FORM = kFormSteadyTau1 when no lattice is at its first iteration after
 // its fields were set and every lattice has τ = 1 (the host knows both).
+// FP32 strips of 64 threads decided at run time without rare forces (τ != 1) take
+// offsets (64 lattices of 6k to 26k cells, τ = 0.8: 41.5 us per iteration, as arrays
+// 45.3), the others arrays (their steady form, one of 1M cells: 27.9 and 24.9).
+template <class S, int NT, bool GEN, int FORM>
+struct BatchStoreOf {
+    using type = S;
+};
+template <class L>
+struct BatchStoreOf<StoreF32T<L>, 64, false, kFormAny> {
+    using type = StoreF32T<L, true>;
+};
 template <class S, int NT, bool GEN, int FORM = kFormAny, bool WAVE = false>
 __global__ void __launch_bounds__(NT) batch_step_kernel(const StepArgs *__restrict__ args,
                                                         const TileRef *__restrict__ tiles,
                                                         int ntiles, int k) {
-    __shared__ MarchSmem<S, NT> sm;
+    using P = typename BatchStoreOf<S, NT, GEN, FORM>::type;
+    __shared__ MarchSmem<P, NT> sm;
     __shared__ StepArgs sa;
     grid_dep_wait();
     for (int e = blockIdx.x; e < ntiles; e += gridDim.x) {
@@ -2168,9 +2180,9 @@ __global__ void __launch_bounds__(NT) batch_step_kernel(const StepArgs *__restri
         const long long done = sa.ctl->step_base + k;
         if (tr.tx >= 0) {
             if constexpr (FORM == kFormSteadyTau1)
-                march_run<S, NT, false, true, GEN, WAVE>(sa, tr.tx, tr.ty, done, sm);
+                march_run<P, NT, false, true, GEN, WAVE>(sa, tr.tx, tr.ty, done, sm);
             else
-                march_tile<S, NT, GEN>(sa, tr.tx, tr.ty, done, sm);
+                march_tile<P, NT, GEN>(sa, tr.tx, tr.ty, done, sm);
         } else if (k > 0 && done <= sa.stop_at)
             reduce_step<NT>(sa, done, sm.redd);
         __syncthreads();
