@@ -553,10 +553,13 @@ constexpr int kBurst = 4096;                  // iterations between records
 constexpr size_t kPartBytes = (size_t)64 << 20;  // of measures a burst keeps
 
 // Cuts the lattices into chunks of one CTA each and returns the iterations K
-// of a launch.  A launch of c CTAs per SM lasts about K max(1, c / r) t + t0:
+// of a launch.  A launch of c CTAs per SM lasts about K max(1, c / r) t + t0 + c l:
 // Float64 t = 2.5 us with CTAs of 128 cells and 1.75 with 64, r = 1 (one CTA keeps
-// an SM's Float64 units busy), FP32 t = 0.9 us and r = 8 (it leaves them idle),
-// t0 = 2 us; larger K need more CTAs, because 6 K of their cells are halo.
+// an SM's Float64 units busy), FP32 t = 0.9 us and r = 6.25 (it leaves them idle),
+// t0 = 2 us, l = 0.15 us (FP32; for its loads and stores, 4 % of a Float64 CTA's
+// time); larger K need more CTAs, because 6 K of their cells are halo.  With FP32 the
+// K this gives are within 2 % of the best of 1 to 20 for 1 to 3000 lattices of 130
+// to 2M cells (2000 of 1000 cells: K = 4 26.9 us per iteration; 2 30.8, 8 30.5).
 int split_lattices(swb1d *b, std::vector<swb::D1Chunk> &out) {
     int sms = 1, dev = 0;
     cudaGetDevice(&dev);
@@ -570,13 +573,14 @@ int split_lattices(swb1d *b, std::vector<swb::D1Chunk> &out) {
     double cost = 1e300;
     for (int nt : {swb::kD1Cells, swb::kD1Cells / 2}) {
         if (nt != swb::kD1Cells && !f64) break;
-        const double t = !f64 ? 0.9 : (nt == swb::kD1Cells ? 2.5 : 1.75), r = f64 ? 1.0 : 8.0;
+        const double t = !f64 ? 0.9 : (nt == swb::kD1Cells ? 2.5 : 1.75), r = f64 ? 1.0 : 6.25;
         for (int K = 1; 6 * K + 8 <= nt; ++K) {
             long long n = 0;
             for (const swb_params &p : b->params) n += pieces(p.Lx, nt, K);
-            const double c = std::max(1.0, std::ceil((double)n / sms) / r) * t + 2.0 / K;
-            if (c < cost) {
-                cost = c;
+            const double us = std::max(1.0, std::ceil((double)n / sms) / r) * t +
+                              (2.0 + (f64 ? 0.0 : 0.15) * (double)n / sms) / K;
+            if (us < cost) {
+                cost = us;
                 best = K;
                 cells = nt;
             }
