@@ -13,6 +13,7 @@ The memory stays the pool's, so ndarray.resize refuses these arrays.
 from __future__ import annotations
 
 import collections
+import math
 import mmap
 import os
 import threading
@@ -84,7 +85,7 @@ def _take(size: int):
 
 def empty(shape) -> np.ndarray:
     """An uninitialised column-major Float64 array."""
-    n = 8 * int(np.prod(shape))
+    n = 8 * math.prod(shape)
     if n < MIN_BYTES:
         return np.empty(shape, dtype=np.float64, order="F")
     mem = _take(-(-n // mmap.PAGESIZE) * mmap.PAGESIZE)
